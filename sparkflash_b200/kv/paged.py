@@ -45,6 +45,8 @@ class PagedKV:
         need, own = -(-rows // PAGE), self.pages[lane]
         if need > self.max_pages:
             raise ValueError(f"{rows} positions are beyond the context of {self.max_pages * PAGE}")
+        if need <= len(own):
+            return
         if need - len(own) > self.pager.free:
             raise PagesExhausted(f"lane {lane} needs {need - len(own)} more pages, {self.pager.free} of {self.n_pages} are free")
         while len(own) < need:
