@@ -24,6 +24,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "k_cache_bf16.cuh"
 #include "k_common.cuh"
 
 namespace sfb {
@@ -186,50 +187,6 @@ __device__ __forceinline__ void at_mark(const AttnTcArgs& a, int slot) {
 __device__ __forceinline__ void at_mark(const AttnTcArgs&, int) {}
 #endif
 
-// ---- cache codes -> bf16 by bit placement ----------------------------------------------------------------------
-// An E4M3 byte shifted into a bf16 (sign to bit 15, the seven exponent|mantissa bits to bits 4..10) is the code's value
-// times 2^-120, subnormal codes included (they land on bf16 subnormals); an E2M1 nibble placed the same way (sign to bit
-// 15, three bits to 6..8) is its value times 2^-126.  Two exact bf16 multiplications by powers of two (the second one
-// carrying the block scale) undo the factor; every intermediate is representable, so the result is the exact product.
-__device__ __forceinline__ uint32_t e4m3x2_to_bf16x2_raw(uint32_t two_bytes_in_high_halves) {
-  // input: byte a in bits 8..15, byte b in bits 24..31
-  const uint32_t t = two_bytes_in_high_halves;
-  return (t & 0x80008000u) | ((t >> 4) & 0x07f007f0u);
-}
-__device__ __forceinline__ uint32_t bf16x2_mul(uint32_t a, uint32_t b) {
-  __nv_bfloat162 r = __hmul2(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
-  return *reinterpret_cast<uint32_t*>(&r);
-}
-__device__ __forceinline__ uint32_t bf16x2_splat(float f) {
-  __nv_bfloat162 r = __float2bfloat162_rn(f);
-  return *reinterpret_cast<uint32_t*>(&r);
-}
-// 16 E4M3 codes (one uint4) with one power-of-two scale -> two uint4 of bf16; m1, m2: splatted bf16 multipliers
-__device__ __forceinline__ void fp8x16_to_bf16(const uint4& v, uint32_t m1, uint32_t m2, uint4& o0, uint4& o1) {
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-  uint32_t r[8];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t lo = __byte_perm(w[i], 0u, 0x1404);   // bytes: [0, b0, 0, b1] -> b0 in bits 8..15, b1 in bits 24..31
-    const uint32_t hi = __byte_perm(w[i], 0u, 0x3424);   // b2, b3
-    r[2 * i] = bf16x2_mul(bf16x2_mul(e4m3x2_to_bf16x2_raw(lo), m1), m2);
-    r[2 * i + 1] = bf16x2_mul(bf16x2_mul(e4m3x2_to_bf16x2_raw(hi), m1), m2);
-  }
-  o0 = make_uint4(r[0], r[1], r[2], r[3]);
-  o1 = make_uint4(r[4], r[5], r[6], r[7]);
-}
-// 8 E2M1 codes (one 32-bit word, element i in nibble i) -> one uint4 of bf16
-__device__ __forceinline__ uint4 fp4x8_to_bf16(uint32_t w, uint32_t m1, uint32_t m2) {
-  uint32_t r[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t x = (w >> (8 * i)) & 0xffu;
-    const uint32_t lanes = (x & 0xfu) | ((x & 0xf0u) << 12);          // nibble 0 in bits 0..3, nibble 1 in bits 16..19
-    const uint32_t raw = ((lanes & 0x00080008u) << 12) | ((lanes & 0x00070007u) << 6);
-    r[i] = bf16x2_mul(bf16x2_mul(raw, m1), m2);
-  }
-  return make_uint4(r[0], r[1], r[2], r[3]);
-}
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -243,12 +200,65 @@ __device__ __forceinline__ void tc_st8(uint32_t taddr, const uint32_t* v) {
                ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
 
+// Second pass of the epilogue for sixteen consecutive dims of one head (two neighbouring lanes share a 32-dim scale block): the inverse rope on the
+// last rd dims and the two-term FP8 copy, both from the staged bf16 rows; packed conversions, 16-byte stores.
+__device__ __forceinline__ void attn_tc_finish(const AttnTcArgs& a, __nv_bfloat16* st_o, uint8_t* st_hi, uint8_t* st_lo, uint8_t* st_sh, uint8_t* st_sl,
+                                               const float2* rope_tab, int sgm, int r0, int seg0) {
+  const int hh = sgm >> 5, seg = sgm & 31;
+  if (!a.out_q && seg < seg0) return;
+  uint4* src = reinterpret_cast<uint4*>(st_o + hh * HD + seg * 16);
+  const uint4 a0 = src[0], a1 = src[1];
+  uint32_t w[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+  if (seg >= seg0) {
+    // inverse rope on the segment's eight (even, odd) pairs, one word each; written back for the bf16 output
+    const float2* rt = &rope_tab[(seg * 16 - r0) >> 1];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const float x = __uint_as_float(w[k] << 16), y = __uint_as_float(w[k] & 0xffff0000u);
+      const float2 c2 = rt[k];
+      w[k] = pack_bf16(__fmaf_rn(x, c2.x, __fmul_rn(y, c2.y)), __fmaf_rn(y, c2.x, -__fmul_rn(x, c2.y)));
+    }
+    src[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    src[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  }
+  if (!a.out_q) return;
+  float o[16];
+  float amax = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    o[2 * k] = __uint_as_float(w[k] << 16);
+    o[2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u);
+    amax = fmaxf(amax, fmaxf(fabsf(o[2 * k]), fabsf(o[2 * k + 1])));      // fmaxf drops a NaN operand: it counts as 0
+  }
+  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+  const uint8_t sc = act_scale_code_fp8(amax);
+  const float inv = bits_f32(((uint32_t)(254 - sc)) << 23);
+  uint32_t hw[4], lw[4];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const float x0 = o[2 * k] * inv, x1 = o[2 * k + 1] * inv;
+    const uint16_t h2 = enc_e4m3x2(x0, x1);
+    uint32_t hf;
+    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(hf) : "h"(h2));
+    const float2 dq = __half22float2(*reinterpret_cast<const __half2*>(&hf));
+    const uint16_t l2 = enc_e4m3x2((x0 - dq.x) * 16.f, (x1 - dq.y) * 16.f);
+    if (k & 1) { hw[k >> 1] |= (uint32_t)h2 << 16; lw[k >> 1] |= (uint32_t)l2 << 16; }
+    else { hw[k >> 1] = h2; lw[k >> 1] = l2; }
+  }
+  *reinterpret_cast<uint4*>(st_hi + hh * HD + seg * 16) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+  *reinterpret_cast<uint4*>(st_lo + hh * HD + seg * 16) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+  if (!(sgm & 1)) {
+    st_sh[hh * (HD / 32) + (seg >> 1)] = sc;
+    st_sl[hh * (HD / 32) + (seg >> 1)] = sc >= 4 ? (uint8_t)(sc - 4) : (uint8_t)0;
+  }
+}
+
 template <int NH>
 struct AttnTcSmem {
   alignas(1024) uint8_t kv[SLABS * SLAB_BYTES];   // 128 keys x 512 dims bf16, eight swizzled slabs
   alignas(1024) uint8_t q[SLABS * NH * 128];      // NH heads x 512 dims bf16
   alignas(1024) uint8_t p[2 * NH * 128];          // NH heads x 128 keys bf16 (two slabs of 64 keys)
-  float sbuf[(NH < 32 ? NH : 32)][KT + 1];        // scores of the tile, head-major: 32 heads per softmax pass
+  float sbuf[NH][KT + 1];                         // scores of the tile, head-major
   alignas(8) float red[THREADS];                  // per (key part, head) partial max / sum; outside the softmax: the row's rope table
   float fac[NH];                                  // per-head rescale of the running accumulator; 1/denominator at the end
   alignas(8) uint64_t bar;                        // score MMAs done (two issuing threads)
@@ -269,13 +279,9 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(AttnTcArgs a) {
   // output: four 128-dim tiles (one issuing thread each).  A thread issues one tcgen05 operation per ~80 cycles whatever its
   // size, and with 32-column MMAs that paced the tile.
   constexpr uint32_t TMEM_COLS = NH * 6 <= 128 ? 128 : (NH * 6 <= 256 ? 256 : 512);
-  // the softmax runs over SH heads at a time (all of them up to 32; two passes for a 64-head group, which halves the
-  // conversions of the key tiles per row against two 32-head CTAs)
-  constexpr int SH = NH < 32 ? NH : 32;
-  constexpr int NPASS = NH / SH;
-  constexpr int PARTS = THREADS / SH;      // key parts per head in the softmax
+  constexpr int PARTS = THREADS / NH;      // key parts per head in the softmax
   constexpr int KPP = KT / PARTS;          // keys per part
-  constexpr int CH = SH / 2;               // score columns per half and pass
+  constexpr int CH = NH / 2;               // score columns per half
   constexpr float LOG2E = 1.4426950408889634f;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int half = tid >> 7, key_slot = tid & 127;
@@ -324,15 +330,12 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(AttnTcArgs a) {
   const int n_sel = a.ckv_q ? a.sel_count[row] : 0;
   const int total = n_win + n_sel;
   const int tiles = (total + KT - 1) / KT;
-  const int my_head = tid % SH, my_part = tid / SH;
-  float m_run[NPASS], l_run[NPASS];        // identical in every thread that shares my_head
-#pragma unroll
-  for (int ps = 0; ps < NPASS; ++ps) { m_run[ps] = -1e30f; l_run[ps] = 0.f; }
+  const int my_head = tid % NH, my_part = tid / NH;
+  float m_run = -1e30f, l_run = 0.f;       // identical in every thread that shares my_head
   uint32_t parity = 0;
   bool ok = true;
   const float sl2 = a.scale * LOG2E;
   const uint32_t M60 = bf16x2_splat(1.152921504606847e18f);      // 2^60
-  const uint32_t M100 = bf16x2_splat(1.2676506002282294e30f);    // 2^100
 
   // the FP4 codes and scales of the NEXT tile's compressed entry are requested while the current tile is multiplied and
   // normalised, so that the gather's trip to L2 / HBM is not on the tile's critical path
@@ -383,13 +386,13 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(AttnTcArgs a) {
         const uint8_t* scb = reinterpret_cast<const uint8_t*>(&sc4);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {          // 32 codes per uint4, two E4M3 scales
+          uint32_t s0, s1;
+          e4m3x2_splat((uint16_t)(scb[2 * i] | (scb[2 * i + 1] << 8)), s0, s1);
           const uint32_t w4[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            // E4M3 scale (exact in bf16) times the 2^26 left over: 2^-126 = 2^-100 2^-26
-            const uint32_t m2 = bf16x2_splat(e4m3_to_f32(scb[2 * i + (j >> 1)]) * 67108864.f);
             const int c = half * 32 + i * 4 + j;
-            *reinterpret_cast<uint4*>(rowp + (c >> 3) * SLAB_BYTES + swz(key_slot, c & 7)) = fp4x8_to_bf16(w4[j], M100, m2);
+            *reinterpret_cast<uint4*>(rowp + (c >> 3) * SLAB_BYTES + swz(key_slot, c & 7)) = fp4x8_to_bf16(w4[j], j < 2 ? s0 : s1);
           }
         }
       } else {
@@ -455,68 +458,63 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(AttnTcArgs a) {
     if (!ok) break;
     tc_fence_after();
     if (tile == 0) at_mark(a, 4);
-    // ---- scores: TMEM (lane = key) -> shared memory, head-major; each half takes half of the pass's head columns ----
+    // ---- scores: TMEM (lane = key) -> shared memory, head-major; each half takes half of the head columns ----
     int any_rescale = 0;
-#pragma unroll 1
-    for (int ps = 0; ps < NPASS; ++ps) {
-      {
-        const bool valid = tile * KT + key_slot < total;
-        if constexpr (CH == 16) {
-          uint32_t v[16], v1[16];
-          tc_ld16(t_s + lane_base + ps * SH + half * CH, v);
-          tc_ld16(t_s + NH + lane_base + ps * SH + half * CH, v1);
-          tc_wait_ld();
+    {
+      const bool valid = tile * KT + key_slot < total;
+      if constexpr (CH == 16) {
+        uint32_t v[16], v1[16];
+        tc_ld16(t_s + lane_base + half * CH, v);
+        tc_ld16(t_s + NH + lane_base + half * CH, v1);
+        tc_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 16; ++j)
-            S.sbuf[half * CH + j][key_slot] = valid ? (__uint_as_float(v[j]) + __uint_as_float(v1[j])) * sl2 : -INFINITY;
-        } else {
-          uint32_t v[8], v1[8];
-          tc_ld8(t_s + lane_base + ps * SH + half * CH, v);
-          tc_ld8(t_s + NH + lane_base + ps * SH + half * CH, v1);
-          tc_wait_ld();
+        for (int j = 0; j < 16; ++j)
+          S.sbuf[half * CH + j][key_slot] = valid ? (__uint_as_float(v[j]) + __uint_as_float(v1[j])) * sl2 : -INFINITY;
+      } else {
+        uint32_t v[8], v1[8];
+        tc_ld8(t_s + lane_base + half * CH, v);
+        tc_ld8(t_s + NH + lane_base + half * CH, v1);
+        tc_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            S.sbuf[half * CH + j][key_slot] = valid ? (__uint_as_float(v[j]) + __uint_as_float(v1[j])) * sl2 : -INFINITY;
-        }
+        for (int j = 0; j < 8; ++j)
+          S.sbuf[half * CH + j][key_slot] = valid ? (__uint_as_float(v[j]) + __uint_as_float(v1[j])) * sl2 : -INFINITY;
       }
-      __syncthreads();
-      // ---- online softmax: thread = (head of the pass, key part) ----
-      float mloc = -INFINITY;
-      const float* srow = &S.sbuf[my_head][my_part * KPP];
-#pragma unroll
-      for (int i = 0; i < KPP; ++i) mloc = fmaxf(mloc, srow[i]);
-      S.red[my_part * SH + my_head] = mloc;
-      __syncthreads();
-      float m_new = m_run[ps];
-#pragma unroll
-      for (int pp = 0; pp < PARTS; ++pp) m_new = fmaxf(m_new, S.red[pp * SH + my_head]);
-      // the reference exponent moves only when the maximum grew by more than 2^8: probabilities up to 256 are as exact in
-      // bf16 as probabilities up to 1, numerator and denominator use the same reference, and the running output then
-      // rarely needs rescaling (a read-modify-write of the whole TMEM accumulator per tile)
-      if (m_new - m_run[ps] <= 8.f) m_new = m_run[ps];
-      const float corr = exp2f(m_run[ps] - m_new);
-      if (corr != 1.f) any_rescale = 1;
-      __syncthreads();                 // everyone has read the maxima before the sums overwrite them
-      float lsum = 0.f;
-      const int gh = ps * SH + my_head;            // head inside the CTA's group
-#pragma unroll
-      for (int i = 0; i < KPP; i += 2) {
-        const float p0 = exp2f(srow[i] - m_new), p1 = exp2f(srow[i + 1] - m_new);
-        const __nv_bfloat162 pb = __floats2bfloat162_rn(p0, p1);
-        lsum += __bfloat162float(pb.x) + __bfloat162float(pb.y);      // the denominator sums what the value contraction multiplies
-        const int key = my_part * KPP + i;
-        *reinterpret_cast<__nv_bfloat162*>(S.p + (key >> 6) * (NH * 128) + swz(gh, (key & 63) >> 3) + (key & 7) * 2) = pb;
-      }
-      S.red[my_part * SH + my_head] = lsum;
-      if (my_part == 0) S.fac[gh] = corr;
-      __syncthreads();
-      float lt = 0.f;
-#pragma unroll
-      for (int pp = 0; pp < PARTS; ++pp) lt += S.red[pp * SH + my_head];
-      l_run[ps] = l_run[ps] * corr + lt;
-      m_run[ps] = m_new;
-      if (NPASS > 1) __syncthreads();    // the next pass overwrites sbuf and red
     }
+    __syncthreads();
+    // ---- online softmax: thread = (head, key part) ----
+    float mloc = -INFINITY;
+    const float* srow = &S.sbuf[my_head][my_part * KPP];
+#pragma unroll
+    for (int i = 0; i < KPP; ++i) mloc = fmaxf(mloc, srow[i]);
+    S.red[my_part * NH + my_head] = mloc;
+    __syncthreads();
+    float m_new = m_run;
+#pragma unroll
+    for (int pp = 0; pp < PARTS; ++pp) m_new = fmaxf(m_new, S.red[pp * NH + my_head]);
+    // the reference exponent moves only when the maximum grew by more than 2^8: probabilities up to 256 are as exact in
+    // bf16 as probabilities up to 1, numerator and denominator use the same reference, and the running output then
+    // rarely needs rescaling (a read-modify-write of the whole TMEM accumulator per tile)
+    if (m_new - m_run <= 8.f) m_new = m_run;
+    const float corr = exp2f(m_run - m_new);
+    if (corr != 1.f) any_rescale = 1;
+    __syncthreads();                 // everyone has read the maxima before the sums overwrite them
+    float lsum = 0.f;
+#pragma unroll
+    for (int i = 0; i < KPP; i += 2) {
+      const float p0 = exp2f(srow[i] - m_new), p1 = exp2f(srow[i + 1] - m_new);
+      const __nv_bfloat162 pb = __floats2bfloat162_rn(p0, p1);
+      lsum += __bfloat162float(pb.x) + __bfloat162float(pb.y);      // the denominator sums what the value contraction multiplies
+      const int key = my_part * KPP + i;
+      *reinterpret_cast<__nv_bfloat162*>(S.p + (key >> 6) * (NH * 128) + swz(my_head, (key & 63) >> 3) + (key & 7) * 2) = pb;
+    }
+    S.red[my_part * NH + my_head] = lsum;
+    if (my_part == 0) S.fac[my_head] = corr;
+    __syncthreads();
+    float lt = 0.f;
+#pragma unroll
+    for (int pp = 0; pp < PARTS; ++pp) lt += S.red[pp * NH + my_head];
+    l_run = l_run * corr + lt;
+    m_run = m_new;
     // ---- rescale the running O^T (lane = dim, column = head): half h owns the 128-dim tiles 2h and 2h + 1 ----
     any_rescale = __syncthreads_or(any_rescale);      // CTA-uniform: did any head's reference exponent move?
     if (tile == 0) at_mark(a, 5);
@@ -563,12 +561,9 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(AttnTcArgs a) {
   if (ok) {
     if (tid < (a.rd >> 1)) rope_tab[tid] = a.rope[(size_t)row * a.rope_stride + tid];      // the last softmax is done with the scratch
     if (my_part == 0) {
-#pragma unroll
-      for (int ps = 0; ps < NPASS; ++ps) {
-        const int ghead = hg * NH + ps * SH + my_head;
-        const float sk = ghead < a.heads ? a.sink[ghead] : 0.f;
-        S.fac[ps * SH + my_head] = 1.f / (l_run[ps] + exp2f(sk * LOG2E - m_run[ps]));
-      }
+      const int ghead = hg * NH + my_head;
+      const float sk = ghead < a.heads ? a.sink[ghead] : 0.f;
+      S.fac[my_head] = 1.f / (l_run + exp2f(sk * LOG2E - m_run));
     }
     __syncthreads();
     const size_t Wd = (size_t)a.heads * HD;
@@ -584,8 +579,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(AttnTcArgs a) {
     __nv_bfloat16* st_o = reinterpret_cast<__nv_bfloat16*>(S.kv);
     uint8_t* st_hi = S.kv + NH * HD * 2;
     uint8_t* st_lo = st_hi + NH * HD;
-    // scale codes of the hi term [NH * 16] and of the lo term: in the query buffer, which nothing reads any more (for a
-    // 64-head group the three staged outputs fill the KV buffer exactly)
+    // scale codes of the hi term [NH * 16] and of the lo term: in the query buffer, which nothing reads any more
     uint8_t* st_sh = S.q;
     uint8_t* st_sl = st_sh + NH * (HD / 32);
     // pass 1: TMEM (lane = dim, column = head) -> bf16 [head][dim] in shared memory
@@ -615,55 +609,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(AttnTcArgs a) {
       __syncthreads();
       at_mark(a, 12);
       const int seg0 = r0 >> 4;                     // first 16-dim segment that carries rope (rd is a multiple of 32)
-      for (int sgm = tid; sgm < NH * 32; sgm += THREADS) {
-        const int hh = sgm >> 5, seg = sgm & 31;
-        if (!a.out_q && seg < seg0) continue;
-        uint4* src = reinterpret_cast<uint4*>(st_o + hh * HD + seg * 16);
-        const uint4 a0 = src[0], a1 = src[1];
-        uint32_t w[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-        if (seg >= seg0) {
-          // inverse rope on the segment's eight (even, odd) pairs, one word each; written back for the bf16 output
-          const float2* rt = &rope_tab[(seg * 16 - r0) >> 1];
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const float x = __uint_as_float(w[k] << 16), y = __uint_as_float(w[k] & 0xffff0000u);
-            const float2 c2 = rt[k];
-            w[k] = pack_bf16(__fmaf_rn(x, c2.x, __fmul_rn(y, c2.y)), __fmaf_rn(y, c2.x, -__fmul_rn(x, c2.y)));
-          }
-          src[0] = make_uint4(w[0], w[1], w[2], w[3]);
-          src[1] = make_uint4(w[4], w[5], w[6], w[7]);
-        }
-        if (!a.out_q) continue;
-        float o[16];
-        float amax = 0.f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          o[2 * k] = __uint_as_float(w[k] << 16);
-          o[2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u);
-          amax = fmaxf(amax, fmaxf(fabsf(o[2 * k]), fabsf(o[2 * k + 1])));      // fmaxf drops a NaN operand: it counts as 0
-        }
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        const uint8_t sc = act_scale_code_fp8(amax);
-        const float inv = bits_f32(((uint32_t)(254 - sc)) << 23);
-        uint32_t hw[4], lw[4];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float x0 = o[2 * k] * inv, x1 = o[2 * k + 1] * inv;
-          const uint16_t h2 = enc_e4m3x2(x0, x1);
-          uint32_t hf;
-          asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(hf) : "h"(h2));
-          const float2 dq = __half22float2(*reinterpret_cast<const __half2*>(&hf));
-          const uint16_t l2 = enc_e4m3x2((x0 - dq.x) * 16.f, (x1 - dq.y) * 16.f);
-          if (k & 1) { hw[k >> 1] |= (uint32_t)h2 << 16; lw[k >> 1] |= (uint32_t)l2 << 16; }
-          else { hw[k >> 1] = h2; lw[k >> 1] = l2; }
-        }
-        *reinterpret_cast<uint4*>(st_hi + hh * HD + seg * 16) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-        *reinterpret_cast<uint4*>(st_lo + hh * HD + seg * 16) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
-        if (!(tid & 1)) {
-          st_sh[hh * (HD / 32) + (seg >> 1)] = sc;
-          st_sl[hh * (HD / 32) + (seg >> 1)] = sc >= 4 ? (uint8_t)(sc - 4) : (uint8_t)0;
-        }
-      }
+      for (int sgm = tid; sgm < NH * 32; sgm += THREADS) attn_tc_finish(a, st_o, st_hi, st_lo, st_sh, st_sl, rope_tab, sgm, r0, seg0);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
@@ -698,6 +644,352 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(AttnTcArgs a) {
   __syncthreads();
   at_mark(a, 7);
   if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);
+}
+
+// ---- 64 heads per CTA ----------------------------------------------------------------------------------------------
+struct AttnTc64Smem {
+  alignas(1024) uint8_t kv[SLABS * SLAB_BYTES];   // 128 keys x 512 dims bf16, eight swizzled slabs; at the end the outputs on their way out
+  alignas(1024) uint8_t q[SLABS * 64 * 128];      // 64 heads x 512 dims bf16; at the end the scale codes
+  alignas(1024) uint8_t p[2 * 64 * 128];          // 64 heads x 128 keys bf16 (two slabs of 64 keys)
+  float redm[8][64], redl[8][64];                 // per (sixteen keys, head): maximum, sum
+  float fac[64];                                  // per-head rescale of the running accumulator; 1/denominator at the end
+  alignas(8) float2 rope[128];                    // (cos, sin) of the row's position
+  alignas(8) uint64_t bar;                        // score MMAs done (two issuing threads)
+  alignas(8) uint64_t bar_pv[4];                  // value MMAs of a 128-dim output tile done
+  uint32_t tmem_base;
+};
+constexpr int THREADS64 = 512;
+
+// grid (groups of 64 heads, rows), sixteen warps.  The arithmetic and its order, hence the bits, are those of attn_tc_kernel (tiles of 128
+// keys, two partial score accumulators of 256 dims, sums over sixteen keys at a time), laid out for 64 heads:
+//   keys     thread = (key of the tile, 128 dims): quarter h = tid / 128 decodes slabs 2h and 2h + 1, and waits only for the value MMAs that
+//            read these two (output tile h), so the next tile's codes are widened under the last value MMAs
+//   scores   S[head, key] = Q K^T with M = 64: a head is a TMEM lane (sixteen per warp quarter), so a thread finds the scores of 32 keys of
+//            one head in its own registers: no transposition through shared memory, one exchange of eight partial maxima and sums per head
+//   values   O^T[dim, head], as in attn_tc_kernel: four issuing threads, one 128-dim tile each
+// Shared memory holds one CTA per SM (K 128 KB, Q 64 KB, P 16 KB), so the phases of a tile follow each other; sixteen warps instead of eight
+// halve each thread's chain of loads, conversions and exponentials.  4,096 rows, 64 heads: a layer of
+// 128 window entries 615 -> 553 us, with 512 compressed ones 1,695 -> 1,358 us (a row: 48 us, of which 7.3 per tile after the first).
+__global__ void __launch_bounds__(THREADS64, 1) attn_tc64_kernel(AttnTcArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  AttnTc64Smem& S = *reinterpret_cast<AttnTc64Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  constexpr float LOG2E = 1.4426950408889634f;
+  constexpr int NH = 64;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int quarter = tid >> 7, key_slot = tid & 127;
+  const int hg = blockIdx.x, row = blockIdx.y;
+
+  at_mark(a, 0);
+  if (tid == 0) {
+    mbar_init(&S.bar, 2);
+    for (int j = 0; j < 4; ++j) mbar_init(&S.bar_pv[j], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    tmem_alloc(&S.tmem_base, 512);
+    tmem_relinquish();
+  }
+  pdl_launch_dependents();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  pdl_wait();
+  at_mark(a, 1);
+  const uint32_t tmem = S.tmem_base;
+  const uint32_t t_s = tmem, t_o = tmem + 256;                            // two score accumulators of 128 columns, four output tiles of 64
+  const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+  const int cg = warp >> 2;                                               // keys [32 cg, +32) of the scores, output tile cg
+  const int head = (warp & 3) * 16 + (lane & 15);                         // of the scores: M = 64 fills lanes 0..15 of each warp quarter
+  const bool owner = lane < 16;
+
+  const int pos = a.row_pos[row], L = a.row_lane[row];
+  const int r0 = HD - a.rd;
+  if (tid < (a.rd >> 1)) S.rope[tid] = a.rope[(size_t)row * a.rope_stride + tid];
+  // queries: asynchronous 16-byte copies into the swizzled K-major tile; they land while the first key tile is decoded
+#pragma unroll
+  for (int i = 0; i < NH * 64 / THREADS64; ++i) {
+    const int idx = tid + i * THREADS64, hh = idx >> 6, c = idx & 63;     // head in group, 8-dim chunk
+    const int ghead = hg * NH + hh;
+    uint8_t* dst = S.q + (c >> 3) * (NH * 128) + swz(hh, c & 7);
+    if (ghead < a.heads) cp_async16(smem_u32(dst), a.q + (size_t)row * a.q_stride + (size_t)ghead * HD + c * 8);
+    else *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  at_mark(a, 2);
+
+  const int w_first = a.win_lo ? a.win_lo[row] : (pos - a.window + 1 > 0 ? pos - a.window + 1 : 0);
+  const int n_win = (a.win_hi ? a.win_hi[row] : pos) - w_first + 1;
+  const int n_sel = a.ckv_q ? a.sel_count[row] : 0;
+  const int total = n_win + n_sel;
+  const int tiles = (total + KT - 1) / KT;
+  float m_run = -1e30f, l_run = 0.f;                                      // of this thread's head, the same in its four owners
+  bool ok = true;
+  const float sl2 = a.scale * LOG2E;
+  const uint32_t M60 = bf16x2_splat(1.152921504606847e18f);      // 2^60
+
+  // codes and scales of the NEXT tile's compressed entry are requested while the current tile is multiplied and normalised
+  uint4 nraw[4];
+  uint2 nsc;
+  bool have_next = false;
+  auto request = [&](int e) {
+    const int id = a.sel[(size_t)row * a.K + (e - n_win)];
+    const uint8_t* kq = a.ckv_q + (size_t)L * a.ckv_lane_q + (size_t)id * (HD / 2) + quarter * 64;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) nraw[i] = *reinterpret_cast<const uint4*>(kq + i * 16);
+    nsc = *reinterpret_cast<const uint2*>(a.ckv_s + (size_t)L * a.ckv_lane_s + (size_t)id * (HD / 16) + quarter * 8);
+  };
+#pragma unroll 1
+  for (int tile = 0; tile < tiles; ++tile) {
+    if (tile > 0) ok = mbar_wait(&S.bar_pv[quarter], (tile - 1) & 1) && ok;      // slabs 2h, 2h + 1 are free
+    // ---- decode dims [128 quarter, +128) of key slot `key_slot` into the bf16 tile ----
+    {
+      const int e = tile * KT + key_slot;
+      uint8_t* rowp = S.kv + quarter * 2 * SLAB_BYTES;
+      if (e < n_win) {
+        const int slot = (w_first + e) % a.ring;
+        const uint8_t* kq = a.win_q + (size_t)L * a.win_lane_q + (size_t)slot * HD + quarter * 128;
+        const uint32_t sc = *reinterpret_cast<const uint32_t*>(a.win_s + (size_t)L * a.win_lane_s + (size_t)slot * (HD / 32) + quarter * 4);
+        uint4 raw[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) raw[i] = *reinterpret_cast<const uint4*>(kq + i * 16);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          // block scale 2^(code - 127) times the 2^60 left over from the raw placement (2^-120 = 2^-60 2^-60)
+          const uint32_t m2 = bf16x2_splat(ue8m0_shifted((uint8_t)(sc >> (8 * (i >> 1))), 60));
+          uint4 o0, o1;
+          fp8x16_to_bf16(raw[i], M60, m2, o0, o1);
+          *reinterpret_cast<uint4*>(rowp + (i >> 2) * SLAB_BYTES + swz(key_slot, (2 * i) & 7)) = o0;
+          *reinterpret_cast<uint4*>(rowp + (i >> 2) * SLAB_BYTES + swz(key_slot, (2 * i + 1) & 7)) = o1;
+        }
+      } else if (e < total) {
+        if (!have_next) request(e);
+        const uint32_t sc4[2] = {nsc.x, nsc.y};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {          // 32 codes per uint4, two E4M3 scales
+          uint32_t s0, s1;
+          e4m3x2_splat((uint16_t)(sc4[i >> 1] >> (16 * (i & 1))), s0, s1);
+          const uint32_t w4[4] = {nraw[i].x, nraw[i].y, nraw[i].z, nraw[i].w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            *reinterpret_cast<uint4*>(rowp + (i >> 1) * SLAB_BYTES + swz(key_slot, (4 * i + j) & 7)) = fp4x8_to_bf16(w4[j], j < 2 ? s0 : s1);
+        }
+      } else {
+        // past the row's last key: zeros, so that the value contraction adds 0 x 0 and never meets stale bits
+        const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int c = 0; c < 16; ++c) *reinterpret_cast<uint4*>(rowp + (c >> 3) * SLAB_BYTES + swz(key_slot, c & 7)) = z;
+      }
+    }
+    {
+      const int en = (tile + 1) * KT + key_slot;      // this thread's entry of the next tile
+      have_next = en >= n_win && en < total;
+      if (have_next) request(en);
+    }
+    if (tile == 0) {
+      // the queries have landed: rope on dims [r0, 512) of every head, in place (one 8-dim chunk per thread and turn)
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+      const int rc = a.rd >> 3;                     // roped chunks per head
+      for (int idx = tid; idx < NH * rc; idx += THREADS64) {
+        const int hh = idx / rc, c = (r0 >> 3) + idx % rc;
+        if (hg * NH + hh >= a.heads) continue;
+        uint4* qp = reinterpret_cast<uint4*>(S.q + (c >> 3) * (NH * 128) + swz(hh, c & 7));
+        uint4 v = *qp;
+        __nv_bfloat162* pr = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 c2 = S.rope[((c * 8 - r0) >> 1) + j];
+          const float x = __bfloat162float(pr[j].x), y = __bfloat162float(pr[j].y);
+          pr[j] = __floats2bfloat162_rn(x * c2.x - y * c2.y, x * c2.y + y * c2.x);
+        }
+        *qp = v;
+      }
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    tc_fence_before();
+    ok = __syncthreads_and(ok ? 1 : 0) != 0;
+    if (!ok) break;
+    if (tile == 0) at_mark(a, 3);
+    // ---- S = Q K^T ----
+    if (warp < 2 && elect_one()) {      // warp 0: slabs 0..3 into S0, warp 1: slabs 4..7 into S1
+      tc_fence_after();
+      const uint32_t idesc = make_idesc(64, 128, 0);
+      const uint32_t kvb = smem_u32(S.kv), qb = smem_u32(S.q);
+      const int s0 = warp * (SLABS / 2);
+#pragma unroll 1
+      for (int s = s0; s < s0 + SLABS / 2; ++s) {
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+          tc_mma_f16(t_s + warp * 128, make_desc(qb + s * (NH * 128) + kk * 32, 1024, 16), make_desc(kvb + s * SLAB_BYTES + kk * 32, 1024, 16),
+                     idesc, ((s - s0) | kk) ? 1u : 0u);
+      }
+      tc_commit(&S.bar);
+    }
+    __syncwarp();
+    ok = mbar_wait(&S.bar, tile & 1);
+    tc_fence_after();
+    if (tile == 0) at_mark(a, 4);
+    // ---- online softmax of 32 keys of one head per owner; part = sixteen keys ----
+    float s[32];
+    {
+      uint32_t v0[32];
+      tc_ld16(t_s + lane_base + cg * 32, v0);
+      tc_ld16(t_s + lane_base + cg * 32 + 16, v0 + 16);
+      uint32_t v1[32];
+      tc_ld16(t_s + 128 + lane_base + cg * 32, v1);
+      tc_ld16(t_s + 128 + lane_base + cg * 32 + 16, v1 + 16);
+      tc_wait_ld();
+      const int left = total - tile * KT - cg * 32;      // keys of these 32 that exist
+#pragma unroll
+      for (int i = 0; i < 32; ++i) s[i] = i < left ? __fmul_rn(__uint_as_float(v0[i]) + __uint_as_float(v1[i]), sl2) : -INFINITY;
+    }
+    float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+    for (int i = 0; i < 32; ++i) mx[i >> 4] = fmaxf(mx[i >> 4], s[i]);
+    if (owner) { S.redm[cg * 2][head] = mx[0]; S.redm[cg * 2 + 1][head] = mx[1]; }
+    tc_fence_before();
+    ok = __syncthreads_and(ok ? 1 : 0) != 0;
+    if (!ok) break;
+    float m_new = m_run;
+#pragma unroll
+    for (int pp = 0; pp < 8; ++pp) m_new = fmaxf(m_new, S.redm[pp][head]);
+    // the reference exponent moves only when the maximum grew by more than 2^8 (see attn_tc_kernel)
+    if (m_new - m_run <= 8.f) m_new = m_run;
+    const float corr = exp2f(m_run - m_new);
+    float lsum[2] = {0.f, 0.f};
+    uint32_t pw[16];
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) {
+      const float p0 = exp2f(s[i] - m_new), p1 = exp2f(s[i + 1] - m_new);
+      const __nv_bfloat162 pb = __floats2bfloat162_rn(p0, p1);
+      lsum[i >> 4] += __bfloat162float(pb.x) + __bfloat162float(pb.y);      // the denominator sums what the value contraction multiplies
+      pw[i >> 1] = *reinterpret_cast<const uint32_t*>(&pb);
+    }
+    if (owner) {
+      S.redl[cg * 2][head] = lsum[0]; S.redl[cg * 2 + 1][head] = lsum[1];
+      if (cg == 0) S.fac[head] = corr;
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        *reinterpret_cast<uint4*>(S.p + (cg >> 1) * (NH * 128) + swz(head, (cg & 1) * 4 + c)) = make_uint4(pw[4 * c], pw[4 * c + 1], pw[4 * c + 2], pw[4 * c + 3]);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    const int any_rescale = __syncthreads_or(corr != 1.f ? 1 : 0);      // did any head's reference exponent move?
+    float lt = 0.f;
+#pragma unroll
+    for (int pp = 0; pp < 8; ++pp) lt += S.redl[pp][head];
+    l_run = l_run * corr + lt;
+    m_run = m_new;
+    if (tile == 0) at_mark(a, 5);
+    // ---- rescale the running O^T (lane = dim, column = head): a warp takes its quarter's lanes of tile cg ----
+    if (tile > 0 && any_rescale) {
+      // every value MMA of the previous tile is done: the warps of each quarter waited for theirs before this tile's keys
+#pragma unroll 1
+      for (int c0 = 0; c0 < NH; c0 += 16) {
+        uint32_t v[16];
+        tc_ld16(t_o + lane_base + cg * NH + c0, v);
+        tc_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * S.fac[c0 + i]);
+        tc_st16(t_o + lane_base + cg * NH + c0, v);
+      }
+      tc_wait_st();
+      tc_fence_before();
+      __syncthreads();
+    }
+    // ---- O^T += V^T P^T ----
+    if (warp < 4 && elect_one()) {      // warp j issues the 128-dim output tile j
+      tc_fence_after();
+      const uint32_t idesc = make_idesc(128, NH, 1);
+      const uint32_t kvb = smem_u32(S.kv), pb = smem_u32(S.p);
+      const int j = warp;
+#pragma unroll
+      for (int t8 = 0; t8 < KT / 16; ++t8)
+        tc_mma_f16(t_o + j * NH, make_desc(kvb + (2 * j) * SLAB_BYTES + t8 * 2048, 1024, SLAB_BYTES),
+                   make_desc(pb + (t8 >> 2) * (NH * 128) + (t8 & 3) * 32, 1024, 16), idesc, (tile > 0 || t8 > 0) ? 1u : 0u);
+      tc_commit(&S.bar_pv[j]);
+    }
+    __syncwarp();
+    if (tile == 0) at_mark(a, 6);
+  }
+  if (ok && tiles > 0) {
+#pragma unroll 1
+    for (int j = 0; j < 4; ++j) ok = mbar_wait(&S.bar_pv[j], (tiles - 1) & 1) && ok;
+  }
+  if (ok && owner && cg == 0) {
+    const int ghead = hg * NH + head;
+    const float sk = ghead < a.heads ? a.sink[ghead] : 0.f;
+    S.fac[head] = 1.f / (l_run + exp2f(sk * LOG2E - m_run));
+  }
+  ok = __syncthreads_and(ok ? 1 : 0) != 0;
+  tc_fence_after();
+  at_mark(a, 8);
+
+  // ---- epilogue: O^T / denominator (sink in the denominator only), inverse rope, bf16 (+ two-term FP8 copy), as in attn_tc_kernel ----
+  if (ok) {
+    const size_t Wd = (size_t)a.heads * HD;
+    int row_hi = row, row_lo = a.n + row;
+    if (a.pair_block > 0) {
+      row_hi = (row / a.pair_block) * 2 * a.pair_block + row % a.pair_block;
+      row_lo = row_hi + a.pair_block;
+    }
+    const int KB = a.heads * (HD / 32);
+    __nv_bfloat16* st_o = reinterpret_cast<__nv_bfloat16*>(S.kv);      // bf16 [64][512], then the two FP8 terms: the KV buffer exactly
+    uint8_t* st_hi = S.kv + NH * HD * 2;
+    uint8_t* st_lo = st_hi + NH * HD;
+    uint8_t* st_sh = S.q;                                              // scale codes of the two terms [64 * 16]
+    uint8_t* st_sl = st_sh + NH * (HD / 32);
+    {
+      const int dim = cg * 128 + (warp & 3) * 32 + lane;
+      uint32_t v[4][16];
+#pragma unroll
+      for (int ch = 0; ch < 4; ++ch) tc_ld16(t_o + lane_base + cg * NH + ch * 16, v[ch]);
+      tc_wait_ld();
+#pragma unroll
+      for (int ch = 0; ch < 4; ++ch)
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          st_o[(ch * 16 + i) * HD + dim] = __float2bfloat16_rn(tiles > 0 ? __uint_as_float(v[ch][i]) * S.fac[ch * 16 + i] : 0.f);
+    }
+    at_mark(a, 11);
+    __syncthreads();
+    at_mark(a, 12);
+    const int seg0 = r0 >> 4;                     // first 16-dim segment that carries rope (rd is a multiple of 32)
+#pragma unroll
+    for (int turn = 0; turn < NH * 32 / THREADS64; ++turn)
+      attn_tc_finish(a, st_o, st_hi, st_lo, st_sh, st_sl, S.rope, tid + turn * THREADS64, r0, seg0);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    at_mark(a, 9);
+    const int head0 = hg * NH;
+    const int nvalid = a.heads - head0 < NH ? a.heads - head0 : NH;        // heads of this group that exist
+    if (nvalid > 0) {
+      if (tid == 0) {
+        bulk_store(a.out + ((size_t)row * a.heads + head0) * HD, smem_u32(st_o), (uint32_t)nvalid * HD * 2);
+        bulk_store_commit_wait_read();
+      } else if (tid == 32 && a.out_q) {
+        bulk_store(a.out_q + (size_t)row_hi * Wd + (size_t)head0 * HD, smem_u32(st_hi), (uint32_t)nvalid * HD);
+        bulk_store_commit_wait_read();
+      } else if (tid == 64 && a.out_q) {
+        bulk_store(a.out_q + (size_t)row_lo * Wd + (size_t)head0 * HD, smem_u32(st_lo), (uint32_t)nvalid * HD);
+        bulk_store_commit_wait_read();
+      }
+      if (a.out_q) {
+        // scale bytes: four k-blocks (one k-atom) of a row are four consecutive bytes of the atom layout
+        for (int wd = tid; wd < nvalid * (HD / 128); wd += THREADS64) {
+          const int kb = head0 * (HD / 32) + wd * 4;
+          *reinterpret_cast<uint32_t*>(a.out_atom + sf_offset(row_hi, kb, KB)) = reinterpret_cast<const uint32_t*>(st_sh)[wd];
+          *reinterpret_cast<uint32_t*>(a.out_atom + sf_offset(row_lo, kb, KB)) = reinterpret_cast<const uint32_t*>(st_sl)[wd];
+        }
+      }
+    }
+  } else if (tid == 0) {
+    status_set(a.status, ST_TIMEOUT, 50, blockIdx.x, blockIdx.y);
+  }
+  at_mark(a, 10);
+  tc_fence_before();
+  __syncthreads();
+  at_mark(a, 7);
+  if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
 }  // namespace sfb
@@ -745,10 +1037,10 @@ int sfb_attn_tc(const void* q, int64_t q_stride, const void* rope, int rope_stri
     if (!done) { cudaFuncSetAttribute(attn_tc_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); done = true; }
     rc = sfb_launch(attn_tc_kernel<32>, dim3(1, n), dim3(atc::THREADS), smem, stream, a);
   } else {       // 64 heads per CTA: a row's key tiles are converted once for all of them
-    const size_t smem = sizeof(AttnTcSmem<64>) + 1024;
+    const size_t smem = sizeof(AttnTc64Smem) + 1024;
     static bool done = false;
-    if (!done) { cudaFuncSetAttribute(attn_tc_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); done = true; }
-    rc = sfb_launch(attn_tc_kernel<64>, dim3((heads + 63) / 64, n), dim3(atc::THREADS), smem, stream, a);
+    if (!done) { cudaFuncSetAttribute(attn_tc64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); done = true; }
+    rc = sfb_launch(attn_tc64_kernel, dim3((heads + 63) / 64, n), dim3(THREADS64), smem, stream, a);
   }
   return (int)rc;
 }

@@ -198,6 +198,33 @@ def test_attention_tc_agrees_with_rows_kernel():
     assert (a.float() - b.float()).abs().max() <= 0.02 * a.float().abs().max()
 
 
+@pytest.mark.parametrize("selected", [0, 1, 127, 128, 129, 512])
+def test_attention_of_64_heads_at_the_edges_of_key_tiles(selected):
+    """Rows whose window and selected entries end inside, at and one past a tile of 128 keys, through the 64-head kernel (70 heads: a second,
+    mostly empty group) and the rows kernel."""
+    from sparkflash_b200.ops import native as N
+    heads = 70
+    c = _attention_case(heads, [0, 126, 127, 128, 800], True, seed=5)
+    cnt = torch.full((5,), selected, dtype=torch.int32)
+    for r in range(5):
+        c["sel"][r, :selected] = torch.arange(selected, dtype=torch.int32) + r
+    dev = "cuda"
+    n, hd, rd = c["n"], c["hd"], c["rd"]
+    rope = torch.zeros(n, 1, rd // 2, 2, dtype=torch.float32, device=dev)
+    N.rope_table([c["invf"].to(dev)], [1], c["pos"].to(dev), rope, n)
+    args = (c["q"].to(dev), heads * hd, rope[:, 0], c["lane"].to(dev), c["pos"].to(dev), c["wq"].to(dev), c["ws"].to(dev),
+            C.pack_nibbles(c["cq"]).to(dev), c["cs"].to(dev), c["sel"].to(dev), cnt.to(dev), c["K"], c["sink"].to(dev))
+    a = torch.zeros(n, heads * hd, dtype=torch.bfloat16, device=dev)
+    b = torch.zeros_like(a)
+    status = torch.zeros(4, dtype=torch.int32, device=dev)
+    N.attn_rows(*args, a, n, heads, hd, rd, c["window"], c["ring"], hd ** -0.5)
+    N.attn_tc(*args, b, n, heads, hd, rd, c["window"], c["ring"], hd ** -0.5, status=status)
+    torch.cuda.synchronize()
+    assert status.tolist()[0] == 0
+    # probabilities in bf16 (2^-8 of each, in numerator and denominator alike) and one rounding of the output each
+    assert (a.float() - b.float()).abs().max() <= 2 ** -6 * a.float().abs().max()
+
+
 def _index_case(n, entries, lanes, seed):
     g = torch.Generator().manual_seed(seed)
     inh, idh, rd = 32, 128, 64
