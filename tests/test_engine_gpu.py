@@ -261,6 +261,55 @@ def test_attention_rows_matches_fp32_reference():
         assert (got - o).abs().max() <= 0.02 * o.abs().max() + 1e-4, (r, (got - o).abs().max(), o.abs().max())
 
 
+@pytest.mark.parametrize("hd,heads,window,selected", [(512, 64, 128, 512), (512, 20, 128, 512), (512, 3, 128, 700), (512, 17, 9, 0), (128, 16, 128, 33),
+                                                      (64, 5, 200, 512), (512, 16, 1, 7)])
+@pytest.mark.parametrize("apart", [0, 1])
+def test_attention_rows_at_the_edges_of_heads_entries_and_chunks(hd, heads, window, selected, apart):
+    """Head groups that are not full, fewer entries than CTAs, more than one chunk of 80 entries per CTA, query rows off 16-byte boundaries.
+    The rotation is a quarter turn, which is exact, so what is left against 64 bits is the rounding of the output to bf16 (8 significant
+    bits: half a unit of the last place is at most 2^-8 of a value) and 32-bit sums and exponentials (below 2^-16 of the largest value)."""
+    from sparkflash_b200.ops import native as N
+    g = torch.Generator().manual_seed(hd + heads + selected)
+    dev, rd, ring, lanes, entries, n = "cuda", 32, 256, 2, 800, 3
+    pos, lane = torch.tensor([900, 40, 3], dtype=torch.int32), torch.tensor([1, 0, 1], dtype=torch.int32)
+    wq, ws = C.act_quant_fp8(torch.randn(lanes, ring, hd, generator=g))
+    cq, cs = C.kv_quant_fp4(torch.randn(lanes, entries, hd, generator=g))
+    K = max(selected, 1)
+    sel = torch.full((n, K), -1, dtype=torch.int32)
+    cnt = torch.tensor([selected, min(selected, 11), 0], dtype=torch.int32)
+    for r in range(n):
+        sel[r, :int(cnt[r])] = torch.randperm(entries, generator=g)[:int(cnt[r])].sort().values.int()
+    q = (torch.randn(n, heads * hd, generator=g) * 2).to(torch.bfloat16)
+    wide = torch.zeros(n, heads * hd + apart, dtype=torch.bfloat16, device=dev)
+    wide[:, apart:] = q.to(dev)
+    rope = torch.tensor([0.0, 1.0], device=dev).repeat(n, rd // 2, 1).contiguous()
+    sink = torch.randn(heads, generator=g)
+    out = torch.zeros(n, heads * hd, dtype=torch.bfloat16, device=dev)
+    out_q = torch.zeros(2 * n, heads * hd, dtype=torch.uint8, device=dev)
+    atom = torch.zeros(C.sf_bytes(128, heads * hd // 32), dtype=torch.uint8, device=dev)
+    N.attn_rows(wide[:, apart:], heads * hd + apart, rope, lane.to(dev), pos.to(dev), wq.to(dev), ws.to(dev), C.pack_nibbles(cq).to(dev),
+                cs.to(dev), sel.to(dev), cnt.to(dev), K, sink.to(dev), out, n, heads, hd, rd, window, ring, hd ** -0.5, out_q=out_q, out_atom=atom)
+    torch.cuda.synchronize()
+    wd, cd = C.act_dequant_fp8(wq, ws).double(), C.kv_dequant_fp4(cq, cs).double()
+
+    def turn(x, sign):
+        y = x.clone()
+        y[..., hd - rd::2], y[..., hd - rd + 1::2] = -sign * x[..., hd - rd + 1::2], sign * x[..., hd - rd::2]
+        return y
+    for r in range(n):
+        p, L = int(pos[r]), int(lane[r])
+        keys = torch.stack([wd[L, t % ring] for t in range(max(0, p - window + 1), p + 1)] + [cd[L, j] for j in sel[r, :int(cnt[r])].tolist()])
+        s = torch.cat([turn(q[r].double().view(heads, hd), 1) @ keys.t() * hd ** -0.5, sink.double()[:, None]], 1)
+        o = turn(torch.softmax(s, -1)[:, :-1] @ keys, -1)
+        got = out[r].cpu().double().view(heads, hd)
+        assert ((got - o).abs() <= 2 ** -8 * o.abs() + 2 ** -16 * o.abs().max()).all(), r
+        # the two-term copy: 3 + 1 significant bits in the high term, as many of the rest in the low one
+        code, scale = C.act_quant_fp8(out[r].cpu().float().view(heads, hd))
+        assert torch.equal(out_q[r].cpu().view(heads, hd), code)
+        val = (C.e4m3_decode(out_q[r].cpu()) + C.e4m3_decode(out_q[n + r].cpu()) / 16).view(heads, hd) * C.ue8m0_decode(scale).repeat_interleave(32, -1)
+        assert ((val - out[r].cpu().float().view(heads, hd)).abs() <= 2 ** -7 * val.abs() + 2 ** -12 * val.abs().max()).all()
+
+
 def test_rows_step_is_batch_invariant_and_graph_replay_is_exact(tiny):
     from sparkflash_b200.models.deepseek_v41 import engine as E
     cfg, ck, w, orc, dw = tiny
