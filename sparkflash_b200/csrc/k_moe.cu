@@ -321,7 +321,7 @@ struct MoePlanArgs {
   const int* ids;        // [n, k] expert id (local; < 0 = not on this rank)
   const float* wts;      // [n, k]
   int n, k, E, shared, S;          // S = segments launched (fixed per row count)
-  int seg;                         // pair slots per segment (16, or 64 for many-row steps)
+  int seg;                         // pair slots per segment (16; 64 or 96 for many-row steps)
   int* seg_expert;       // [S]  -1 unused, -2 shared expert
   int* seg_count;        // [S]
   float* seg_weight;     // [S*16]
@@ -469,7 +469,7 @@ extern "C" int sfb_expert_remap(void* ids, int n, int lo, int count, cudaStream_
 
 extern "C" int sfb_moe_plan(const void* ids, const void* wts, int n, int k, int E, int shared, int S, int seg, void* seg_expert, void* seg_count,
                             void* seg_weight, void* seg_token, void* pair_pos, cudaStream_t stream) {
-  if (E > 4096 || (seg != 16 && seg != 64)) return (int)cudaErrorInvalidValue;
+  if (E > 4096 || (seg != 16 && seg != 64 && seg != 96)) return (int)cudaErrorInvalidValue;
   sfb::MoePlanArgs a{(const int*)ids, (const float*)wts, n, k, E, shared, S, seg, (int*)seg_expert, (int*)seg_count, (float*)seg_weight,
                      (int*)seg_token, (int*)pair_pos};
   return (int)sfb::sfb_launch(sfb::moe_plan_kernel, dim3(1), dim3(512), (size_t)(3 * E + 1) * sizeof(int), stream, a);

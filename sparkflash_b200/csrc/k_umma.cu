@@ -1271,23 +1271,27 @@ umma_gateup_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_const
   if (warp == 1) tmem_dealloc(tmem, TMEM_COLS);
 }
 
-// ---- persistent grouped gate/up for wide (64-pair) segments --------------------------------------------------------------
+// ---- persistent grouped gate/up for wide segments (NP = 64 or 96 pairs) --------------------------------------------------------------
 // One CTA per SM walks over (column tile of the intermediate width, segment) pairs.  While the four epilogue warps turn one
 // tile's accumulators into FP8 activations (SwiGLU, routing weight, re-quantisation: 14 of a one-tile CTA's 48 us), the
 // producer and the two MMA-issuing threads are already in the next tile's main loop on the other accumulator set.  The
 // arithmetic, its order and the output bits are those of umma_gateup_kernel<2, 64>.
-constexpr int PG_STAGES = 5;
-constexpr int PG_NP = 64;
-struct UmmaGateupPersistSmem {
-  alignas(1024) uint8_t a[PG_STAGES][2][UM_A_BYTES];
-  alignas(1024) uint8_t b[PG_STAGES][PG_NP * UM_BK];
-  alignas(1024) uint8_t sq[PG_NP * 128];          // the tile's FP8 codes on their way out, pair-major
+// Bound by what comes out of L2 and by the operand reads of the MMAs from shared memory, both of which the weight tiles dominate: every segment
+// reads its expert's weights again.  96 pairs are what two accumulator sets of two tiles leave room for in TMEM (4 x 96 columns and the
+// scale factors); 128 would leave one set and put the epilogue back on the critical path.  4,096 rows over 64 experts
+// (384 pairs each): 768 us against 836 with 64 pairs.
+template <int NP> constexpr int PG_STAGES = NP == 64 ? 5 : 4;      // what shared memory holds
+template <int NP> struct UmmaGateupPersistSmem {
+  static constexpr int ST = PG_STAGES<NP>;
+  alignas(1024) uint8_t a[ST][2][UM_A_BYTES];
+  alignas(1024) uint8_t b[ST][NP * UM_BK];
+  alignas(1024) uint8_t sq[NP * 128];          // the tile's FP8 codes on their way out, pair-major
   alignas(128) uint8_t ssf[512];                  // and its scale atom
-  alignas(128) uint8_t sfa[PG_STAGES][2][512];
-  alignas(128) uint8_t sfb[PG_STAGES][512];
-  alignas(8) uint64_t full[PG_STAGES];
-  alignas(8) uint64_t empty[PG_STAGES];
-  alignas(8) uint64_t sfready[PG_STAGES][2];      // the stage's scale factors are in TMEM (one barrier per accumulator)
+  alignas(128) uint8_t sfa[ST][2][512];
+  alignas(128) uint8_t sfb[ST][512];
+  alignas(8) uint64_t full[ST];
+  alignas(8) uint64_t empty[ST];
+  alignas(8) uint64_t sfready[ST][2];      // the stage's scale factors are in TMEM (one barrier per accumulator)
   alignas(8) uint64_t acc_full[2];
   alignas(8) uint64_t acc_empty[2];
   uint32_t tmem_base;
@@ -1300,19 +1304,21 @@ struct UmmaGateupPersistSmem {
 // shipped choice); the copier threads date from roles entered by lane index, where seven operations per k-step paced the loop.
 constexpr int PG_THREADS = 288;
 
+template <int NP>
 __global__ void __launch_bounds__(PG_THREADS, 1)
 umma_gateup_persistent_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapA2,
                               const __grid_constant__ CUtensorMap tmapB, UmmaArgs a, int n_tiles, int n_segs, int copier_threads) {
   extern __shared__ uint8_t smem_raw[];
-  using Smem = UmmaGateupPersistSmem;
+  using Smem = UmmaGateupPersistSmem<NP>;
   Smem& S = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  constexpr int NP = PG_NP;
+  constexpr int ST = PG_STAGES<NP>;
+  static_assert(4 * NP + 4 * 4 * ST <= 512, "two accumulator sets and the scale factors fit TMEM");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int il = a.inter;
   const int nks = (a.d + UM_BK - 1) / UM_BK;
   const int total = n_tiles * n_segs;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < PG_STAGES; ++s) {
+    for (int s = 0; s < ST; ++s) {
       mbar_init(&S.full[s], 1); mbar_init(&S.empty[s], 2);
       mbar_init(&S.sfready[s][0], 1); mbar_init(&S.sfready[s][1], 1);
     }
@@ -1332,8 +1338,8 @@ umma_gateup_persistent_kernel(const __grid_constant__ CUtensorMap tmapA, const _
   pdl_wait();
   const uint32_t tmem = S.tmem_base;
   // scale factors: one 4-column slot per stage and operand, so a slot is rewritten only after the MMAs of the stage's previous
-  // use are done (the producer refills the stage only then): gate weights 256.., gate's activation copy 276.., up 296.., 316..
-  const uint32_t t_sfg = tmem + 256, t_sfb = tmem + 276, t_sfu = tmem + 296, t_sfb2 = tmem + 316;
+  // use are done (the producer refills the stage only then), behind the accumulators: gate weights, gate's activation copy, up, its copy
+  const uint32_t t_sfg = tmem + 4 * NP, t_sfb = t_sfg + 4 * ST, t_sfu = t_sfb + 4 * ST, t_sfb2 = t_sfu + 4 * ST;
 
   if (warp == 0) {
     if (elect_one()) {
@@ -1360,8 +1366,8 @@ umma_gateup_persistent_kernel(const __grid_constant__ CUtensorMap tmapA, const _
         const uint8_t* sfb = a.sfb + (size_t)seg * a.katoms_b * 512;
         const uint32_t stage_tx = 2 * (a_fp4 ? UM_A_BYTES / 2 : UM_A_BYTES) + NP * UM_BK + 3 * 512;
         for (int i = 0; i < nks; ++i, ++it) {
-          const int s = it % PG_STAGES;
-          if (it >= PG_STAGES && !mbar_wait(&S.empty[s], ((it / PG_STAGES) - 1) & 1)) { S.fail = 1; break; }
+          const int s = it % ST;
+          if (it >= ST && !mbar_wait(&S.empty[s], ((it / ST) - 1) & 1)) { S.fail = 1; break; }
           mbar_expect_tx(&S.full[s], stage_tx);
           tma_load_2d(S.a[s][0], ma, i * UM_BK, row_g, &S.full[s]);
           tma_load_2d(S.a[s][1], ma, i * UM_BK, row_u, &S.full[s]);
@@ -1389,12 +1395,12 @@ umma_gateup_persistent_kernel(const __grid_constant__ CUtensorMap tmapA, const _
         if (lt >= 2 && !mbar_wait(&S.acc_empty[buf], ((lt >> 1) - 1) & 1)) { S.fail = 3; break; }
         if (SFB_MARKS_ON) c_acc += clock64() - w0;
         tc_fence_after();
-        const uint32_t t_d = tmem + (uint32_t)buf * 128 + (h ? NP : 0);
+        const uint32_t t_d = tmem + (uint32_t)buf * (2 * NP) + (h ? NP : 0);
         bool ok = true;
         for (int i = 0; i < nks; ++i, ++it) {
-          const int s = it % PG_STAGES;
+          const int s = it % ST;
           const long long w1 = SFB_MARKS_ON ? clock64() : 0;
-          if (!mbar_wait(copier_threads ? &S.sfready[s][h] : &S.full[s], (it / PG_STAGES) & 1)) { S.fail = 2; ok = false; break; }
+          if (!mbar_wait(copier_threads ? &S.sfready[s][h] : &S.full[s], (it / ST) & 1)) { S.fail = 2; ok = false; break; }
           if (SFB_MARKS_ON) c_full += clock64() - w1;
           tc_fence_after();
           const uint32_t sl = (uint32_t)s * 4;
@@ -1431,8 +1437,8 @@ umma_gateup_persistent_kernel(const __grid_constant__ CUtensorMap tmapA, const _
         if (a.seg_expert[t / n_tiles] == -1) continue;
         bool ok = true;
         for (int i = 0; i < nks; ++i, ++it) {
-          const int s = it % PG_STAGES;
-          if (!mbar_wait(&S.full[s], (it / PG_STAGES) & 1)) { S.fail = 4; ok = false; break; }
+          const int s = it % ST;
+          if (!mbar_wait(&S.full[s], (it / ST) & 1)) { S.fail = 4; ok = false; break; }
           tc_fence_after();
           tc_cp_sf(t_sa + (uint32_t)s * 4, make_desc(smem_u32(S.sfa[s][h]), 128, 0, 0));
           tc_cp_sf(t_sb + (uint32_t)s * 4, make_desc(smem_u32(S.sfb[s]), 128, 0, 0));
@@ -1469,7 +1475,7 @@ umma_gateup_persistent_kernel(const __grid_constant__ CUtensorMap tmapA, const _
       tc_fence_after();
       reinterpret_cast<uint32_t*>(S.ssf)[q * 32 + lane] = 0x7f7f7f7fu;      // rows past the segment's pairs: scale 1
       asm volatile("bar.sync 1, 128;" ::: "memory");
-      const uint32_t t_g = tmem + (uint32_t)buf * 128, t_u = t_g + NP;
+      const uint32_t t_g = tmem + (uint32_t)buf * (2 * NP), t_u = t_g + NP;
       const int col = tile * 128 + q * 32 + lane;
 #pragma unroll 1
       for (int c0 = 0; c0 < NP && c0 < ncol; c0 += 16) {
@@ -1754,19 +1760,21 @@ umma_down_persistent_kernel(const __grid_constant__ CUtensorMap tmapA, const __g
 // ---- persistent grouped down projection, two column tiles per work item --------------------------------------------------------
 // The one-tile form above carries 8 KB of weights and 8 KB of activations per stage, so only half of its ring of stages is
 // HBM traffic.  Here a work item is a PAIR of neighbouring column tiles of one segment: both weight tiles share the stage's
-// activation tile (stage = 2 x 16 KB + 8 KB, five stages: 80 KB of weights in flight per SM instead of 56), each has its own
+// activation tile (64 pairs: stage = 2 x 16 KB + 8 KB, five stages: 80 KB of weights in flight per SM instead of 56), each has its own
 // accumulator (two sets of two) and the fp32 tiles leave through a 16 KB staging buffer, 32 pair rows at a time.  Arithmetic,
-// order and output bits are those of the one-tile kernels.
-constexpr int PD2_STAGES = 5;
-struct UmmaDownPersist2Smem {
-  alignas(1024) uint8_t a[PD2_STAGES][2][UM_A_BYTES];
-  alignas(1024) uint8_t b[PD2_STAGES][PD_NP * UM_BK];
+// order and output bits are those of the one-tile kernels.  Segments of 64 or 96 pairs, as in the gate/up kernel.  4,096 rows: 449 us
+// against 472.
+template <int NP> constexpr int PD2_STAGES = NP == 64 ? 5 : 4;      // what shared memory holds
+template <int NP> struct UmmaDownPersist2Smem {
+  static constexpr int ST = PD2_STAGES<NP>;
+  alignas(1024) uint8_t a[ST][2][UM_A_BYTES];
+  alignas(1024) uint8_t b[ST][NP * UM_BK];
   alignas(1024) float outf[32 * 128];              // 32 pair rows of one tile on their way out
-  alignas(128) uint8_t sfa[PD2_STAGES][2][512];
-  alignas(128) uint8_t sfb[PD2_STAGES][512];
-  alignas(8) uint64_t full[PD2_STAGES];
-  alignas(8) uint64_t empty[PD2_STAGES];
-  alignas(8) uint64_t sfready[PD2_STAGES];
+  alignas(128) uint8_t sfa[ST][2][512];
+  alignas(128) uint8_t sfb[ST][512];
+  alignas(8) uint64_t full[ST];
+  alignas(8) uint64_t empty[ST];
+  alignas(8) uint64_t sfready[ST];
   alignas(8) uint64_t acc_full[2];
   alignas(8) uint64_t acc_empty[2];
   uint32_t tmem_base;
@@ -1774,13 +1782,15 @@ struct UmmaDownPersist2Smem {
   volatile int ep_ok;
 };
 
+template <int NP>
 __global__ void __launch_bounds__(PD_THREADS, 1)
 umma_down_persistent2_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapA2,
                              const __grid_constant__ CUtensorMap tmapB, UmmaArgs a, int n_tile_pairs, int n_segs) {
   extern __shared__ uint8_t smem_raw[];
-  using Smem = UmmaDownPersist2Smem;
+  using Smem = UmmaDownPersist2Smem<NP>;
   Smem& S = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  constexpr int NP = PD_NP, ST = PD2_STAGES;
+  constexpr int ST = PD2_STAGES<NP>, ROUNDS = NP / 32;
+  static_assert(NP % 32 == 0 && 4 * NP + 3 * 4 * ST <= 512, "two accumulator sets and the scale factors fit TMEM");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nks = (a.inter + UM_BK - 1) / UM_BK;
   const int total = n_tile_pairs * n_segs;
@@ -1801,8 +1811,8 @@ umma_down_persistent2_kernel(const __grid_constant__ CUtensorMap tmapA, const __
   tc_fence_after();
   pdl_wait();
   const uint32_t tmem = S.tmem_base;
-  // accumulators: set b at columns 128 b (tile 0) and 128 b + 64 (tile 1); scale-factor slots per stage and operand from 256
-  const uint32_t t_sfa0 = tmem + 256, t_sfa1 = tmem + 288, t_sfb = tmem + 320;
+  // accumulators: set b at columns 2 NP b (tile 0) and 2 NP b + NP (tile 1); scale-factor slots per stage and operand behind them
+  const uint32_t t_sfa0 = tmem + 4 * NP, t_sfa1 = t_sfa0 + 4 * ST, t_sfb = t_sfa1 + 4 * ST;
 
   if (warp == 0) {
     if (elect_one()) {
@@ -1850,7 +1860,7 @@ umma_down_persistent2_kernel(const __grid_constant__ CUtensorMap tmapA, const __
         const int buf = lt & 1;
         if (lt >= 2 && !mbar_wait(&S.acc_empty[buf], ((lt >> 1) - 1) & 1)) { S.fail = 3; break; }
         tc_fence_after();
-        const uint32_t t_acc = tmem + (uint32_t)buf * 128;
+        const uint32_t t_acc = tmem + (uint32_t)buf * (2 * NP);
         bool ok = true;
         for (int i = 0; i < nks; ++i, ++it) {
           const int s = it % ST;
@@ -1908,13 +1918,13 @@ umma_down_persistent2_kernel(const __grid_constant__ CUtensorMap tmapA, const __
       asm volatile("bar.sync 1, 128;" ::: "memory");
       if (!S.ep_ok) break;
       tc_fence_after();
-      // four rounds: (tile 0, pairs 0..31), (tile 0, pairs 32..63), (tile 1, ...); a round whose pairs do not exist is skipped
+      // rounds of 32 pairs of tile 0, then of tile 1; a round whose pairs do not exist is skipped
 #pragma unroll 1
-      for (int h = 0; h < 4; ++h) {
-        const int j = h >> 1, p0 = (h & 1) * 32;
+      for (int h = 0; h < 2 * ROUNDS; ++h) {
+        const int j = h / ROUNDS, p0 = (h % ROUNDS) * 32;
         if (p0 >= nv) continue;                    // CTA-uniform
         uint32_t v[2][16];
-        const uint32_t t_acc = tmem + (uint32_t)buf * 128 + (uint32_t)j * NP + p0;
+        const uint32_t t_acc = tmem + (uint32_t)buf * (2 * NP) + (uint32_t)j * NP + p0;
         tc_ld16(t_acc + ((uint32_t)(q * 32) << 16), v[0]);
         tc_ld16(t_acc + ((uint32_t)(q * 32) << 16) + 16, v[1]);
         tc_wait_ld();
@@ -2337,6 +2347,30 @@ int sfb_umma_down(const void* tmapA, const void* tmapA2, const void* tmapB, cons
 
 }  // extern "C"
 
+static int sm_count() {
+  static int sms = 0;
+  if (!sms) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
+  return sms;
+}
+template <int NP>
+static int launch_gateup_persistent(const CUtensorMap* mA, const CUtensorMap* mA2, const void* tmapB, const UmmaArgs& a, int segments, cudaStream_t stream) {
+  const size_t smem = sizeof(UmmaGateupPersistSmem<NP>) + 1024;
+  static bool done = false;
+  if (!done) { cudaFuncSetAttribute(umma_gateup_persistent_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); done = true; }
+  const int tiles = a.inter / 128, total = tiles * segments, sms = sm_count();
+  return (int)sfb_launch(umma_gateup_persistent_kernel<NP>, dim3(total < sms ? total : sms), dim3(PG_THREADS), smem, stream, *mA, *mA2,
+                         *(const CUtensorMap*)tmapB, a, tiles, segments, g_tune[2] == 7 ? 1 : 0);
+}
+template <int NP>
+static int launch_down_persistent2(const void* tmapA, const void* tmapA2, const void* tmapB, const UmmaArgs& a, int segments, cudaStream_t stream) {
+  const size_t smem = sizeof(UmmaDownPersist2Smem<NP>) + 1024;
+  static bool done = false;
+  if (!done) { cudaFuncSetAttribute(umma_down_persistent2_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); done = true; }
+  const int pairs = a.d / 256, total = pairs * segments, sms = sm_count();
+  return (int)sfb_launch(umma_down_persistent2_kernel<NP>, dim3(total < sms ? total : sms), dim3(PD_THREADS), smem, stream, *(const CUtensorMap*)tmapA,
+                         *(const CUtensorMap*)(tmapA2 ? tmapA2 : tmapA), *(const CUtensorMap*)tmapB, a, pairs, segments);
+}
+
 extern "C" {
 
 // Grouped MoE (rows sorted by expert, see csrc/k_moe.cu moe_plan): gate/up over `segments` segments of up to 16 pairs.
@@ -2344,7 +2378,7 @@ extern "C" {
 int sfb_umma_gate_up_grouped(const void* tmapA, const void* tmapA2, const void* tmapB, const void* sfa, const void* sfa2, const void* sfb,
                              const int* seg_expert, const int* seg_count, const float* seg_weight, void* act_q, void* act_sf, int segments,
                              int d, int inter, float limit, int seg_size, void* status, cudaStream_t stream) {
-  if (inter % 128 || d % 32 || segments < 1 || (seg_size != 16 && seg_size != 64)) return refuse_args();
+  if (inter % 128 || d % 32 || segments < 1 || (seg_size != 16 && seg_size != 64 && seg_size != 96)) return refuse_args();
   UmmaArgs a{};
   a.sfa = (const uint8_t*)sfa; a.sfa2 = (const uint8_t*)sfa2; a.katoms_a = (d / 32 + 3) / 4; a.sfb = (const uint8_t*)sfb; a.katoms_b = a.katoms_a;
   a.a_fp4 = 1; a.top_k = 0; a.slots = 1; a.inter = inter; a.d = d; a.act_q = (uint8_t*)act_q; a.act_sf = (uint8_t*)act_sf; a.limit = limit;
@@ -2366,17 +2400,10 @@ int sfb_umma_gate_up_grouped(const void* tmapA, const void* tmapA2, const void* 
     return (int)sfb_launch(umma_gateup_kernel<5, 64>, dim3(inter / 128, segments, 1), dim3(GU_THREADS), smem, stream, *mA, *mA2,
                            *(const CUtensorMap*)tmapB, a);
   }
+  if (seg_size == 96) return act_sf ? launch_gateup_persistent<96>(mA, mA2, tmapB, a, segments, stream) : refuse_args();
   // many wide segments: the persistent kernel (g_tune[6]: 1 = never, 2 = whenever the shape allows)
-  if (seg_size == 64 && inter % 128 == 0 && act_sf && g_tune[6] != 1 && (g_tune[6] == 2 || (inter / 128) * segments >= 296)) {
-    static int sms = 0;
-    if (!sms) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
-    const size_t smem = sizeof(UmmaGateupPersistSmem) + 1024;
-    static bool done = false;
-    if (!done) { cudaFuncSetAttribute(umma_gateup_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); done = true; }
-    const int total = (inter / 128) * segments;
-    return (int)sfb_launch(umma_gateup_persistent_kernel, dim3(total < sms ? total : sms), dim3(PG_THREADS), smem, stream, *mA, *mA2,
-                           *(const CUtensorMap*)tmapB, a, inter / 128, segments, g_tune[2] == 7 ? 1 : 0);
-  }
+  if (seg_size == 64 && inter % 128 == 0 && act_sf && g_tune[6] != 1 && (g_tune[6] == 2 || (inter / 128) * segments >= 296))
+    return launch_gateup_persistent<64>(mA, mA2, tmapB, a, segments, stream);
   if (seg_size == 64) {      // segments of up to 64 pairs: two 2-stage CTAs per SM (a stage holds 32 KiB of weights and 8 KiB of tokens)
     const size_t smem64 = sizeof(UmmaSmem<64, 2, 2>) + 1024;
     static bool done64 = false;
@@ -2403,25 +2430,23 @@ int sfb_umma_gate_up_grouped(const void* tmapA, const void* tmapA2, const void* 
 int sfb_umma_down_grouped(const void* tmapA, const void* tmapA2, const void* tmapB, const void* sfa, const void* sfa2, const void* sfb,
                           const int* seg_expert, const int* seg_count, float* out_f, int segments, int d, int inter, int seg_size,
                           void* status, cudaStream_t stream) {
-  if (d % 128 || inter % 128 || segments < 1 || (seg_size != 16 && seg_size != 64)) return refuse_args();
+  if (d % 128 || inter % 128 || segments < 1 || (seg_size != 16 && seg_size != 64 && seg_size != 96)) return refuse_args();
   UmmaArgs a{};
   a.sfa = (const uint8_t*)sfa; a.sfa2 = (const uint8_t*)sfa2; a.katoms_a = (inter / 32 + 3) / 4; a.sfb = (const uint8_t*)sfb; a.katoms_b = a.katoms_a;
   a.a_fp4 = 1; a.mode = UM_DOWN_GROUPED; a.inter = inter; a.d = d; a.out_f = out_f; a.out_stride = d; a.seg_expert = seg_expert;
   a.seg_count = seg_count; a.status = (Status*)status; a.splits = 1;
+  if (seg_size == 96) {      // the caller cuts such segments only where the two-tile kernel can take them
+    if (d % 256 || g_push.n || g_gather.n) return refuse_args();
+    apply_marks(a);
+    return launch_down_persistent2<96>(tmapA, tmapA2, tmapB, a, segments, stream);
+  }
   // many (column tile, segment) pairs: one persistent CTA per SM ([7]: 0 this rule, 1 never, 2 whenever the shape allows)
   if (seg_size == 64 && g_push.n == 0 && g_gather.n == 0 && g_tune[7] != 1 && (g_tune[7] >= 2 || (d / 128) * segments >= 296)) {
     apply_marks(a);
+    if ((d / 128) % 2 == 0 && g_tune[7] != 3)      // pairs of column tiles sharing the activation tile ([7] = 3: one tile per item)
+      return launch_down_persistent2<64>(tmapA, tmapA2, tmapB, a, segments, stream);
     static int sms = 0;
     if (!sms) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
-    if ((d / 128) % 2 == 0 && g_tune[7] != 3) {      // pairs of column tiles sharing the activation tile ([7] = 3: one tile per item)
-      const int total2 = (d / 256) * segments;
-      const size_t smem2 = sizeof(UmmaDownPersist2Smem) + 1024;
-      static bool done2 = false;
-      if (!done2) { cudaFuncSetAttribute(umma_down_persistent2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2); done2 = true; }
-      return (int)sfb_launch(umma_down_persistent2_kernel, dim3(total2 < sms ? total2 : sms), dim3(PD_THREADS), smem2, stream,
-                             *(const CUtensorMap*)tmapA, *(const CUtensorMap*)(tmapA2 ? tmapA2 : tmapA), *(const CUtensorMap*)tmapB, a,
-                             d / 256, segments);
-    }
     const int total = (d / 128) * segments;
     const size_t smem = sizeof(UmmaDownPersistSmem) + 1024;
     static bool done = false;

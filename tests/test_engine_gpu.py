@@ -749,6 +749,22 @@ def test_wide_moe_segments_and_the_persistent_kernels_give_the_bits_of_16_pair_s
     assert torch.equal(outs[2], outs[3])
 
 
+@pytest.mark.parametrize("rows", [5, 96, 97, 128])
+def test_moe_segments_of_96_pairs_give_the_bits_of_16_pair_segments(tiny, rows):
+    """The shared expert's rows fill one segment, or end a row before or after its border; the routed experts' segments are never full."""
+    from sparkflash_b200.models.deepseek_v41 import engine as E
+    cfg, ck, w, orc, dw = tiny
+    prompt, outs = _prompt(cfg, rows, seed=29), []
+    for wide, pairs in ((10 ** 6, 128), (4, 0)):
+        e = E.Engine(dw, max_lanes=2, max_context=256, max_rows=128, arm="tc", use_graphs=False, keep_logits=True)
+        e.GROUP_WIDE_ROWS, e.GROUP_WIDER_PAIRS = wide, pairs
+        assert e._group_size(rows, cfg.top_k, cfg.n_routed_experts) == (16 if pairs else 96)
+        e.step(prompt, [0] * rows, list(range(rows)))
+        e.check_status()
+        outs.append(e.logits[:rows].clone())
+    assert torch.equal(*outs)
+
+
 def test_guard_bands_stay_intact_over_decode_and_chunk_steps_and_report_a_changed_band(tiny):
     """Every device buffer of a guarded engine sits between two 256-byte bands of a fixed pattern: steps of every kind leave
     them intact (no kernel writes outside its buffers), and a band changed from the host is reported with the allocation's
