@@ -657,7 +657,10 @@ class Engine:
         P = n * k
         return min(P, E_local + P // seg) + (n + seg - 1) // seg
 
-    GROUP_WIDE_ROWS = 512   # from this many rows on, segments hold up to 64 pairs (an expert's weights serve four times the rows)
+    # From this many rows on, segments hold up to 64 pairs: an expert's weights then serve four times the rows, and the persistent kernels run.
+    # Steps of four layers over 64 / 128 experts, 16 pairs against 64: 64 rows 2.78 / 3.20 ms against 2.86 / 3.10, 100 rows 2.64 / 3.16 against
+    # 2.52 / 2.99, 200 rows 2.83 / 3.34 against 2.37 / 3.00, 500 rows 4.60 / 5.10 against 3.24 / 3.99.
+    GROUP_WIDE_ROWS = 100
     # From this many pairs per expert on, 96: at 384 pairs gate/up takes 768 us instead of 836 and down 449 instead of 472; at 73 pairs, where one
     # segment of 96 replaces two of 64, both read the weights from HBM at the same pace (222 / 225 and 130 / 128 us), and between 96 and 128 both
     # sizes need two segments, the wider ones with a third more operand reads.

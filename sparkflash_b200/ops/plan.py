@@ -192,7 +192,7 @@ class KernelResolver:
 MANY_ROWS = 128            # above: token-tiled GEMMs, bf16-GEMM coefficients, one-block-per-row fold
 TC_ATTENTION_ROWS = 64     # above: attention on tcgen05 (a tolerance arm)
 GROUP_MIN_ROWS = 4         # from here on the experts run grouped by expert
-GROUP_WIDE_ROWS = 512      # from here on segments hold up to 64 pairs (96 where experts have more: Engine._group_size)
+GROUP_WIDE_ROWS = 100      # from here on segments hold up to 64 pairs (96 where experts have more: Engine._group_size)
 HEAD_TC_MIN_ROWS = 1
 SELECT_LONG_ENTRIES = 32768   # rows longer than this (and few rows) use the chunked select
 
