@@ -664,12 +664,13 @@ constexpr int THREADS64 = 512;
 // keys, two partial score accumulators of 256 dims, sums over sixteen keys at a time), laid out for 64 heads:
 //   keys     thread = (key of the tile, 128 dims): quarter h = tid / 128 decodes slabs 2h and 2h + 1, and waits only for the value MMAs that
 //            read these two (output tile h), so the next tile's codes are widened under the last value MMAs
-//   scores   S[head, key] = Q K^T with M = 64: a head is a TMEM lane (sixteen per warp quarter), so a thread finds the scores of 32 keys of
-//            one head in its own registers: no transposition through shared memory, one exchange of eight partial maxima and sums per head
+//   scores   S[head, key] = Q K^T with M = 64: a head is a TMEM lane (sixteen per warp quarter), so the scores of 32 keys
+//            of a head lie in one thread's registers, half of which go to the lane sixteen on: no transposition through shared memory, one
+//            exchange of eight partial maxima and sums per head
 //   values   O^T[dim, head], as in attn_tc_kernel: four issuing threads, one 128-dim tile each
 // Shared memory holds one CTA per SM (K 128 KB, Q 64 KB, P 16 KB), so the phases of a tile follow each other; sixteen warps instead of eight
 // halve each thread's chain of loads, conversions and exponentials.  4,096 rows, 64 heads: a layer of
-// 128 window entries 615 -> 553 us, with 512 compressed ones 1,695 -> 1,358 us (a row: 48 us, of which 7.3 per tile after the first).
+// 128 window entries 615 -> 545 us, with 512 compressed ones 1,695 -> 1,267 us (553 and 1,358 with sixteen lanes of a warp in the softmax).
 __global__ void __launch_bounds__(THREADS64, 1) attn_tc64_kernel(AttnTcArgs a) {
   extern __shared__ uint8_t smem_raw[];
   AttnTc64Smem& S = *reinterpret_cast<AttnTc64Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -700,7 +701,7 @@ __global__ void __launch_bounds__(THREADS64, 1) attn_tc64_kernel(AttnTcArgs a) {
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
   const int cg = warp >> 2;                                               // keys [32 cg, +32) of the scores, output tile cg
   const int head = (warp & 3) * 16 + (lane & 15);                         // of the scores: M = 64 fills lanes 0..15 of each warp quarter
-  const bool owner = lane < 16;
+  const int part = cg * 2 + (lane >> 4);                                  // sixteen keys of the tile
 
   const int pos = a.row_pos[row], L = a.row_lane[row];
   const int r0 = HD - a.rd;
@@ -722,7 +723,7 @@ __global__ void __launch_bounds__(THREADS64, 1) attn_tc64_kernel(AttnTcArgs a) {
   const int n_sel = a.ckv_q ? a.sel_count[row] : 0;
   const int total = n_win + n_sel;
   const int tiles = (total + KT - 1) / KT;
-  float m_run = -1e30f, l_run = 0.f;                                      // of this thread's head, the same in its four owners
+  float m_run = -1e30f, l_run = 0.f;                                      // of this thread's head, the same in its eight threads
   bool ok = true;
   const float sl2 = a.scale * LOG2E;
   const uint32_t M60 = bf16x2_splat(1.152921504606847e18f);      // 2^60
@@ -829,24 +830,28 @@ __global__ void __launch_bounds__(THREADS64, 1) attn_tc64_kernel(AttnTcArgs a) {
     ok = mbar_wait(&S.bar, tile & 1);
     tc_fence_after();
     if (tile == 0) at_mark(a, 4);
-    // ---- online softmax of 32 keys of one head per owner; part = sixteen keys ----
-    float s[32];
+    // ---- online softmax: a lane takes sixteen keys (a part) of one head.  The scores of a warp's 32 keys lie in lanes 0..15; the later
+    // sixteen go to the other half of the warp ----
+    float s[16];
     {
-      uint32_t v0[32];
+      uint32_t v0[32], v1[32];
       tc_ld16(t_s + lane_base + cg * 32, v0);
       tc_ld16(t_s + lane_base + cg * 32 + 16, v0 + 16);
-      uint32_t v1[32];
       tc_ld16(t_s + 128 + lane_base + cg * 32, v1);
       tc_ld16(t_s + 128 + lane_base + cg * 32 + 16, v1 + 16);
       tc_wait_ld();
-      const int left = total - tile * KT - cg * 32;      // keys of these 32 that exist
+      const int left = total - tile * KT - part * 16;      // keys of these sixteen that exist
 #pragma unroll
-      for (int i = 0; i < 32; ++i) s[i] = i < left ? __fmul_rn(__uint_as_float(v0[i]) + __uint_as_float(v1[i]), sl2) : -INFINITY;
+      for (int i = 0; i < 16; ++i) {
+        const float near = __uint_as_float(v0[i]) + __uint_as_float(v1[i]);
+        const float far = __shfl_sync(0xffffffffu, __uint_as_float(v0[16 + i]) + __uint_as_float(v1[16 + i]), lane & 15);
+        s[i] = i < left ? __fmul_rn(lane < 16 ? near : far, sl2) : -INFINITY;
+      }
     }
-    float mx[2] = {-INFINITY, -INFINITY};
+    float mx = -INFINITY;
 #pragma unroll
-    for (int i = 0; i < 32; ++i) mx[i >> 4] = fmaxf(mx[i >> 4], s[i]);
-    if (owner) { S.redm[cg * 2][head] = mx[0]; S.redm[cg * 2 + 1][head] = mx[1]; }
+    for (int i = 0; i < 16; ++i) mx = fmaxf(mx, s[i]);
+    S.redm[part][head] = mx;
     tc_fence_before();
     ok = __syncthreads_and(ok ? 1 : 0) != 0;
     if (!ok) break;
@@ -856,22 +861,20 @@ __global__ void __launch_bounds__(THREADS64, 1) attn_tc64_kernel(AttnTcArgs a) {
     // the reference exponent moves only when the maximum grew by more than 2^8 (see attn_tc_kernel)
     if (m_new - m_run <= 8.f) m_new = m_run;
     const float corr = exp2f(m_run - m_new);
-    float lsum[2] = {0.f, 0.f};
-    uint32_t pw[16];
+    float lsum = 0.f;
+    uint32_t pw[8];
 #pragma unroll
-    for (int i = 0; i < 32; i += 2) {
+    for (int i = 0; i < 16; i += 2) {
       const float p0 = exp2f(s[i] - m_new), p1 = exp2f(s[i + 1] - m_new);
       const __nv_bfloat162 pb = __floats2bfloat162_rn(p0, p1);
-      lsum[i >> 4] += __bfloat162float(pb.x) + __bfloat162float(pb.y);      // the denominator sums what the value contraction multiplies
+      lsum += __bfloat162float(pb.x) + __bfloat162float(pb.y);      // the denominator sums what the value contraction multiplies
       pw[i >> 1] = *reinterpret_cast<const uint32_t*>(&pb);
     }
-    if (owner) {
-      S.redl[cg * 2][head] = lsum[0]; S.redl[cg * 2 + 1][head] = lsum[1];
-      if (cg == 0) S.fac[head] = corr;
+    S.redl[part][head] = lsum;
+    if (part == 0) S.fac[head] = corr;
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
-        *reinterpret_cast<uint4*>(S.p + (cg >> 1) * (NH * 128) + swz(head, (cg & 1) * 4 + c)) = make_uint4(pw[4 * c], pw[4 * c + 1], pw[4 * c + 2], pw[4 * c + 3]);
-    }
+    for (int c = 0; c < 2; ++c)
+      *reinterpret_cast<uint4*>(S.p + (part >> 2) * (NH * 128) + swz(head, (part & 3) * 2 + c)) = make_uint4(pw[4 * c], pw[4 * c + 1], pw[4 * c + 2], pw[4 * c + 3]);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     const int any_rescale = __syncthreads_or(corr != 1.f ? 1 : 0);      // did any head's reference exponent move?
     float lt = 0.f;
@@ -915,7 +918,7 @@ __global__ void __launch_bounds__(THREADS64, 1) attn_tc64_kernel(AttnTcArgs a) {
 #pragma unroll 1
     for (int j = 0; j < 4; ++j) ok = mbar_wait(&S.bar_pv[j], (tiles - 1) & 1) && ok;
   }
-  if (ok && owner && cg == 0) {
+  if (ok && part == 0) {
     const int ghead = hg * NH + head;
     const float sk = ghead < a.heads ? a.sink[ghead] : 0.f;
     S.fac[head] = 1.f / (l_run + exp2f(sk * LOG2E - m_run));
