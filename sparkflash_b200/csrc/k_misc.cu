@@ -45,15 +45,42 @@ __global__ void __launch_bounds__(256) markov_bias_kernel(float* logits, const _
 }
 
 // tap[row, :] = bf16(mean over copies of h[row, c, :])
-__global__ void tap_mean_kernel(const __nv_bfloat16* h, __nv_bfloat16* tap, int64_t tap_stride, int hc, int d) {
+// V consecutive elements per thread (eight where rows lie on 16-byte boundaries).  Bound by memory: hc copies in, one mean out; 4,096 rows of 5,120,
+// four copies: 93 us an element per thread, 35 so.
+template <int V>
+__global__ void __launch_bounds__(128) tap_mean_kernel(const __nv_bfloat16* h, __nv_bfloat16* tap, int64_t tap_stride, int hc, int d) {
   pdl_launch_dependents();
   pdl_wait();
   const int row = blockIdx.y;
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
+  const int col = (blockIdx.x * blockDim.x + threadIdx.x) * V;
   if (col >= d) return;
-  float s = 0.f;
-  for (int c = 0; c < hc; ++c) s += bf16_to_f(h[((size_t)row * hc + c) * d + col]);
-  tap[(size_t)row * tap_stride + col] = __float2bfloat16_rn(s / (float)hc);
+  float s[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) s[i] = 0.f;
+#pragma unroll 4
+  for (int c = 0; c < hc; ++c) {
+    const __nv_bfloat16* p = h + ((size_t)row * hc + c) * d + col;
+    if constexpr (V == 8) {
+      const uint4 v = *reinterpret_cast<const uint4*>(p);
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { s[2 * i] += __uint_as_float(w[i] << 16); s[2 * i + 1] += __uint_as_float(w[i] & 0xffff0000u); }
+    } else {
+      s[0] += bf16_to_f(*p);
+    }
+  }
+  __nv_bfloat16* o = tap + (size_t)row * tap_stride + col;
+  if constexpr (V == 8) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __nv_bfloat162 t = __floats2bfloat162_rn(s[2 * i] / (float)hc, s[2 * i + 1] / (float)hc);
+      w[i] = *reinterpret_cast<const uint32_t*>(&t);
+    }
+    *reinterpret_cast<uint4*>(o) = make_uint4(w[0], w[1], w[2], w[3]);
+  } else {
+    *o = __float2bfloat16_rn(s[0] / (float)hc);
+  }
 }
 
 // rope[row, v, p] = (cos, sin)(angle) with angle = ((pos / ratio_v) * ratio_v) * inv_freq_v[p], evaluated in
@@ -204,8 +231,9 @@ int sfb_prefetch_experts(const void* base, int64_t stride, int64_t bytes, const 
 }
 
 int sfb_tap_mean(const void* h, void* tap, int64_t tap_stride, int n, int hc, int d, cudaStream_t stream) {
-  return (int)sfb_launch(tap_mean_kernel, dim3((d + 255) / 256, n), dim3(256), 0, stream, (const __nv_bfloat16*)h,
-                         (__nv_bfloat16*)tap, tap_stride, hc, d);
+  if (d % 8 == 0 && tap_stride % 8 == 0 && (uintptr_t)h % 16 == 0 && (uintptr_t)tap % 16 == 0)
+    return (int)sfb_launch(tap_mean_kernel<8>, dim3((d + 1023) / 1024, n), dim3(128), 0, stream, (const __nv_bfloat16*)h, (__nv_bfloat16*)tap, tap_stride, hc, d);
+  return (int)sfb_launch(tap_mean_kernel<1>, dim3((d + 127) / 128, n), dim3(128), 0, stream, (const __nv_bfloat16*)h, (__nv_bfloat16*)tap, tap_stride, hc, d);
 }
 
 // kind: 0 fp8 bytes, 1 fp4 bytes (count = bytes), 2 bf16 elements, 3 f32 elements
