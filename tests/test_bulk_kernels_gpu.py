@@ -225,6 +225,30 @@ def test_attention_of_64_heads_at_the_edges_of_key_tiles(selected):
     assert (a.float() - b.float()).abs().max() <= 2 ** -6 * a.float().abs().max()
 
 
+@pytest.mark.parametrize("n,k,E,seg", [(1, 6, 64, 16), (42, 6, 64, 16), (43, 6, 64, 16), (100, 6, 64, 64), (777, 6, 5, 64), (1000, 2, 300, 96), (3, 1, 1, 16)])
+def test_expert_plan_gives_every_pair_a_place(n, k, E, seg):
+    """Up to 256 pairs by one block in pair order, more by a cluster; experts that are not here (-1), unused experts, the shared expert's rows."""
+    from sparkflash_b200.ops import native as N
+    g, dev = torch.Generator().manual_seed(n + E), "cuda"
+    ids = torch.randint(-1, E, (n, k), generator=g).int()
+    w, S = torch.rand(n, k, generator=g), min(n * k, E + n * k // seg) + -(-n // seg)
+    expert, count, token, pos = (torch.full((m,), 7, dtype=torch.int32, device=dev) for m in (S, S, S * seg, n * (k + 1)))
+    weight = torch.full((S * seg,), 7.0, device=dev)
+    N.moe_plan(ids.to(dev), w.to(dev), n, k, E, True, S, expert, count, weight, token, pos, seg=seg)
+    expert, count, token, pos, weight = expert.cpu(), count.cpu(), token.cpu(), pos.cpu().view(n, k + 1).long(), weight.cpu()
+    here = torch.cat([ids >= 0, torch.ones(n, 1, dtype=torch.bool)], 1)
+    assert (pos[~here] == -1).all() and pos[here].unique().numel() == here.sum()
+    assert (token[pos[here]] == torch.arange(n)[:, None].expand(n, k + 1)[here]).all()
+    assert (expert[pos[here] // seg] == torch.cat([ids, torch.full((n, 1), -2)], 1)[here]).all()
+    assert (weight[pos[here]] == torch.cat([w, torch.ones(n, 1)], 1)[here]).all()
+    used = token.view(S, seg) >= 0
+    assert (used.sum(1) == count).all() and (used.int().diff(dim=1) <= 0).all() and (count[expert == -1] == 0).all()      # filled from the front
+    assert (weight.view(S, seg)[~used] == 0).all()
+    if n * k <= 256:
+        order = [sorted(pos[:, :k][ids == e].tolist()) == pos[:, :k][ids == e].tolist() for e in range(E)]
+        assert all(order)
+
+
 def _index_case(n, entries, lanes, seed):
     g = torch.Generator().manual_seed(seed)
     inh, idh, rd = 32, 128, 64
