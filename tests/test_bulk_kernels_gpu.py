@@ -98,6 +98,40 @@ def test_two_term_block_layout_matches_per_block_launches():
     assert torch.equal(C.prepared_to_scales(oq_atom.cpu(), n, groups * N_ // 32), rs)
 
 
+@pytest.mark.parametrize("n", [577, 640, 700])
+def test_persistent_pair_gemm_gives_the_bits_of_the_tiles(n):
+    """296 tiles and more run on one persistent CTA per SM; the first 64 rows, 32 tiles, do not."""
+    from sparkflash_b200.ops import native as N
+    dev, groups, N_, K = "cuda", 8, 512, 640
+    g = torch.Generator().manual_seed(n)
+    q, s = C.weight_quant_fp8_block32(torch.randn(groups * N_, K, generator=g) * 0.05)
+    sfa, x = C.scales_to_prepared(s, groups * N_, 32).to(dev), torch.randn(n, groups * K, generator=g).to(torch.bfloat16).to(dev)
+    nblk, KB, KBo = (n + 63) // 64, groups * K // 32, groups * N_ // 32
+    xq = torch.zeros(nblk * 128, groups * K, dtype=torch.uint8, device=dev)
+    atom, block = torch.full((C.sf_bytes(nblk * 128, KB),), 127, dtype=torch.uint8, device=dev), C.sf_bytes(128, KB)
+    for b in range(nblk):
+        N.quant_rows(x[64 * b:], xq[128 * b:], None, atom[b * block:], min(64, n - 64 * b), groups * K, split=True, split_off=64)
+    ta = N.TensorMap(q.to(dev).contiguous(), groups * N_, K, K, 128)
+    tiles = N_ // 128 * groups * nblk
+    scratch, tickets = torch.zeros(tiles * 128 * 128, device=dev), torch.zeros(tiles, dtype=torch.int32, device=dev)
+    status = torch.zeros(4, dtype=torch.int32, device=dev)
+
+    def run(first, rows):
+        out = torch.full((rows, groups * N_), 9.0, dtype=torch.bfloat16, device=dev)
+        oq = torch.zeros(rows, groups * N_, dtype=torch.uint8, device=dev)
+        oa = torch.full((C.sf_bytes(rows, KBo),), 127, dtype=torch.uint8, device=dev)
+        tb = N.TensorMap(xq[2 * first:], 128 * -(-rows // 64), groups * K, groups * K, 128)
+        N.umma_pair_bulk(ta, tb, sfa, atom[first // 64 * block:], rows, N_, K, groups=groups, scratch=scratch, tickets=tickets, out_b=out, out_q=oq,
+                         out_q_atom=oa, status=status)
+        return out.cpu(), oq.cpu(), C.prepared_to_scales(oa.cpu(), rows, KBo)
+    whole = run(0, n)
+    for b in range(nblk):
+        m = min(64, n - 64 * b)
+        for w, p in zip(whole, run(64 * b, m)):
+            assert torch.equal(w[64 * b:64 * b + m], p), b
+    assert status.tolist()[0] == 0
+
+
 def _attention_case(heads, rows, with_compressed, seed):
     from sparkflash_b200.models.deepseek_v41 import oracle as O
     from sparkflash_b200.config import full_config
