@@ -152,7 +152,7 @@ struct AttnTcArgs {
   const int* sel_count;     // [n]
   int K;
   const float* sink;        // [heads]
-  __nv_bfloat16* out;       // [n, heads*512]
+  __nv_bfloat16* out;       // [n, heads*512], or null where only the two-term copy is wanted
   uint8_t* out_q;           // optional two-term FP8 copy in blocks of 2*pair_block rows: hi rows then lo rows of each block
   uint8_t* out_atom;        // its scale atoms (128 rows per atom block)
   int pair_block;           // rows per block of the two-term copy (64), or 0: hi rows [0,n), lo rows [n,2n) as the rows kernel
@@ -218,8 +218,7 @@ __device__ __forceinline__ void attn_tc_finish(const AttnTcArgs& a, __nv_bfloat1
       const float2 c2 = rt[k];
       w[k] = pack_bf16(__fmaf_rn(x, c2.x, __fmul_rn(y, c2.y)), __fmaf_rn(y, c2.x, -__fmul_rn(x, c2.y)));
     }
-    src[0] = make_uint4(w[0], w[1], w[2], w[3]);
-    src[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    if (a.out) { src[0] = make_uint4(w[0], w[1], w[2], w[3]); src[1] = make_uint4(w[4], w[5], w[6], w[7]); }
   }
   if (!a.out_q) return;
   float o[16];
@@ -617,7 +616,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(AttnTcArgs a) {
     const int head0 = hg * NH;
     const int nvalid = a.heads - head0 < NH ? a.heads - head0 : NH;        // heads of this group that exist
     if (nvalid > 0) {
-      if (tid == 0) {
+      if (tid == 0 && a.out) {
         bulk_store(a.out + ((size_t)row * a.heads + head0) * HD, smem_u32(st_o), (uint32_t)nvalid * HD * 2);
         bulk_store_commit_wait_read();
       } else if (tid == 32 && a.out_q) {
@@ -966,7 +965,7 @@ __global__ void __launch_bounds__(THREADS64, 1) attn_tc64_kernel(AttnTcArgs a) {
     const int head0 = hg * NH;
     const int nvalid = a.heads - head0 < NH ? a.heads - head0 : NH;        // heads of this group that exist
     if (nvalid > 0) {
-      if (tid == 0) {
+      if (tid == 0 && a.out) {
         bulk_store(a.out + ((size_t)row * a.heads + head0) * HD, smem_u32(st_o), (uint32_t)nvalid * HD * 2);
         bulk_store_commit_wait_read();
       } else if (tid == 32 && a.out_q) {
@@ -1010,14 +1009,14 @@ int sfb_attn_set_marks(void* buf, int cap_ctas) {
   return 0;
 }
 
-// Same arguments as sfb_attn_rows_range plus the layout of the two-term copy (pair_block) and the status word.
+// Same arguments as sfb_attn_rows_range plus the layout of the two-term copy (pair_block) and the status word; out may be null beside out_q.
 // hd must be 512; rd a multiple of 32.  Heads are processed in groups of 64 (16 or 32 when the rank holds at most that many).
 int sfb_attn_tc(const void* q, int64_t q_stride, const void* rope, int rope_stride, const int* row_lane, const int* row_pos,
                 const void* win_q, const void* win_s, int64_t win_lane_q, int64_t win_lane_s, const void* ckv_q, const void* ckv_s,
                 int64_t ckv_lane_q, int64_t ckv_lane_s, const int* sel, const int* sel_count, int K, const float* sink, void* out,
                 void* out_q, void* out_atom, int pair_block, int n, int heads, int hd, int rd, int window, int ring, float scale,
                 const int* win_lo, const int* win_hi, void* status, cudaStream_t stream) {
-  if (hd != atc::HD || rd % 32 || rd > 256 || n < 1 || heads < 1 || (q_stride % 8)) return (int)cudaErrorInvalidValue;
+  if (hd != atc::HD || rd % 32 || rd > 256 || n < 1 || heads < 1 || (q_stride % 8) || (!out && !out_q)) return (int)cudaErrorInvalidValue;
   AttnTcArgs a{};
   a.q = (const __nv_bfloat16*)q; a.q_stride = q_stride; a.rope = (const float2*)rope; a.rope_stride = rope_stride;
   a.row_lane = row_lane; a.row_pos = row_pos; a.win_q = (const uint8_t*)win_q; a.win_s = (const uint8_t*)win_s;

@@ -559,13 +559,14 @@ class Engine:
         # rows of the staging buffers and its own scale-atom block; everything before (and the expert pass after) sees all rows.
         if n > 64 and tc_wo_a and tc_wo_b and hd == 512 and self.bulk_attention:
             # many rows: attention on tcgen05 (a tolerance arm: the probabilities enter the value contraction as bf16), its
-            # two-term FP8 copy in blocks of 64 hi | 64 lo rows, and one launch each for the two output projections
+            # two-term FP8 copy in blocks of 64 hi | 64 lo rows - all that the projections read: the bf16 rows, as many bytes again, are
+            # written for a debugging run only - and one launch each for the two output projections
             tcb = self.tcb
             self._arm_marks("attn")
             N.attn_tc(self.qfull, self.qfull.stride(0), invf, self.row_lane, self.row_pos, kv.win_q[l], kv.win_s[l],
                       kv.ckv_q[owner] if has_c else None, kv.ckv_s[owner] if has_c else None,
                       self.sel if has_c else None, self.sel_cnt if has_c else None, cfg.index_topk, L.sink,
-                      self.attn_out, n, self.hl, hd, rd, cfg.window, kv.ring, hd ** -0.5, out_q=tcb.ao_q, out_atom=tcb.ao_atom,
+                      self.attn_out if self.debug is not None else None, n, self.hl, hd, rd, cfg.window, kv.ring, hd ** -0.5, out_q=tcb.ao_q, out_atom=tcb.ao_atom,
                       pair_block=64, win_lo=win[0] if win else None, win_hi=win[1] if win else None, status=self.status); self._k()
             tba = tcb.bmap(tcb.ao_q, 128 * tcb.nblk, self.hl * hd, 128)
             self._arm_marks("wo_a")

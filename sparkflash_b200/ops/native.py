@@ -468,7 +468,7 @@ def umma_bf16(tmap_a, tmap_b, n, N, K, *, splits=1, scratch=None, tickets=None, 
 
 def attn_tc(q, q_stride, rope, row_lane, row_pos, win_q, win_s, ckv_q, ckv_s, sel, sel_count, K, sink, out, n, heads,
             hd, rd, window, ring, scale, out_q=None, out_atom=None, pair_block=0, win_lo=None, win_hi=None, status=None):
-    """Rows attention on tcgen05 (csrc/k_attn_tc.cu); arguments as ``attn_rows``.  ``pair_block`` > 0: the two-term FP8
+    """Rows attention on tcgen05 (csrc/k_attn_tc.cu); arguments as ``attn_rows``; ``out`` may be None beside ``out_q``.  ``pair_block`` > 0: the two-term FP8
     copy is laid out in blocks of 2 * pair_block buffer rows (hi rows then lo rows of pair_block logical rows)."""
     code = lib().sfb_attn_tc(
         _p(q), c_int64(q_stride), _p(rope), c_int(rope.stride(0) // 2), _p(row_lane), _p(row_pos), _p(win_q), _p(win_s),
