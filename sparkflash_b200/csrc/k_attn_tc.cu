@@ -13,7 +13,8 @@
 // cache's exact values; P is rounded to bf16 for the second contraction (the CUDA-core rows kernel keeps it in
 // fp32: this kernel is a tolerance arm, not a bit-exact one).  Softmax is online over tiles of 128 keys: the
 // score tile goes TMEM -> registers -> shared memory (transposed), threads then own heads, and the running
-// accumulator in TMEM is rescaled per column when a head's maximum moves.  The sink enters the denominator only.
+// accumulator in TMEM is rescaled per column when a head's maximum moves.  More than 32 heads: attn_tc64_kernel below, the same
+// arithmetic laid out for 64 heads per CTA.  The sink enters the denominator only.
 // Query RoPE on load, inverse RoPE on the output's rope slice, optional two-term FP8 copy for the wo_a GEMM.
 //
 // No cluster, no multicast; every mbarrier wait is bounded and reports through the status word.
@@ -1010,7 +1011,7 @@ int sfb_attn_set_marks(void* buf, int cap_ctas) {
 }
 
 // Same arguments as sfb_attn_rows_range plus the layout of the two-term copy (pair_block) and the status word; out may be null beside out_q.
-// hd must be 512; rd a multiple of 32.  Heads are processed in groups of 64 (16 or 32 when the rank holds at most that many).
+// hd must be 512; rd a multiple of 32.  Heads are processed in groups of 64 (attn_tc64_kernel), or all at once when the rank holds at most 16 or 32.
 int sfb_attn_tc(const void* q, int64_t q_stride, const void* rope, int rope_stride, const int* row_lane, const int* row_pos,
                 const void* win_q, const void* win_s, int64_t win_lane_q, int64_t win_lane_s, const void* ckv_q, const void* ckv_s,
                 int64_t ckv_lane_q, int64_t ckv_lane_s, const int* sel, const int* sel_count, int K, const float* sink, void* out,
