@@ -76,6 +76,8 @@ class Step:
     tensor-core arm needs, how many they are, and every tile's page offset among them; head: ``head_rows`` (None = all rows, in order)."""
 
     single = False            # every segment is one row (a decode step)
+    whole = False             # every row has a head, in order
+    graph: tuple | None = None      # key of the captured step that serves this one; where it exists, the arrays above are left out
     taps: list | None = None  # debug: collects the residual after every layer run
 
     def single_rows(self, tc: bool):
@@ -247,7 +249,8 @@ class LayeredEngine:
 
     def _stage(self, segs, advs, heads, temps, seeds, replay: bool | None = None):
         """Fill the pinned index buffer, copy it to the device once, and return the Step over it.  ``replay``: a captured step will do, one that
-        samples (True) or does not; where there is one, it holds the buffer's places itself and the Step stays without them.
+        samples (True) or does not.  The Step of one row per lane, all with a head, then has its ``graph``; where that has been captured, it holds
+        the buffer's places itself and the Step stays without them.
 
         Whole arrays are written at a time and a replayed step makes no views: a portion has thousands of rows, and the device waits for
         this buffer (Fanodra at width 2,048, portion of 4,096 rows: 5.40 -> 4.86 ms per step; Gudutar, 64 decoded rows: 778 -> 683 us)."""
@@ -281,7 +284,7 @@ class LayeredEngine:
         elif heads and max(heads) >= n:
             raise IndexError("list index out of range")
         s.nhead = len(hrows)
-        all_heads = len(hrows) == n and hrows == list(range(n))
+        s.whole = all_heads = len(hrows) == n and hrows == list(range(n))
         put("seed", 0 if seeds is None else [w for i in heads for w in _words(seeds[i])], 2 * len(heads))      # first: 8-byte aligned
         put("temp", 0 if temps is None else [_float_bits(temps[i]) for i in heads], len(heads))
         hpos, rows_tok, rows_pos, rows_lane = put("hpos", None, len(heads)), put("tokens", None, n), put("row_pos", None, n), put("row_lane", None, n)
@@ -345,8 +348,10 @@ class LayeredEngine:
         if self._event is not None:
             self._event.record()
         s.pages = _bucket(s.max_pos // PAGE + 1)
-        if replay is not None and s.single and all_heads and (n, s.pages, replay) in self.graphs:
-            return s
+        if replay is not None and s.single and all_heads:
+            s.graph = (n, s.pages, replay)
+            if s.graph in self.graphs:
+                return s
         s.short_rows = s.short_segs = s.head_rows = None
         for name, view in zip(names, self._meta[:at].split(sizes)):
             setattr(s, name, view)
@@ -376,9 +381,8 @@ class LayeredEngine:
         graphs = self.use_graphs and not masks and self.tap_layers is None
         s = self._stage(segs, advs, heads, temperature, seeds, bool(sample) if graphs else None)
         mask = self._stage_masks(masks, heads) if masks else None
-        whole = head is True or (len(heads) == n and heads == list(range(n)))
-        if s.single and whole and graphs:
-            self._replay(s, sample)
+        if s.graph is not None:
+            self._replay(s, bool(sample))
         else:
             self._run(s, sample, mask)
         for (lane, p0, toks, _), adv in zip(segs, advs):
@@ -387,7 +391,7 @@ class LayeredEngine:
             return self.best_id[:len(heads)] if sample and heads else None if not sync else torch.zeros((n,), dtype=torch.int32)
         self._out[:len(heads)].copy_(self.best_id[:len(heads)], non_blocking=True)
         torch.cuda.current_stream().synchronize()
-        if whole:
+        if s.whole:
             out = self._out[:n].clone()
         else:
             out = torch.zeros((n,), dtype=torch.int32)
@@ -407,7 +411,7 @@ class LayeredEngine:
     def _replay(self, s: Step, sample: bool) -> None:
         """Decode steps: one CUDA graph per (rows, context bucket).  The index buffer is packed the same way for the same row
         count, and a repeated step writes what it wrote before, so the warm-up run, the capture and the replay agree."""
-        key = (s.n, s.pages, sample)
+        key = s.graph
         g = self.graphs.get(key)
         if g is None:
             from ..runtime.segments import recording
