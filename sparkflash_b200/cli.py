@@ -145,8 +145,8 @@ def _plan(args) -> int:
     from .ops import plan as OP
     cfg = CF.full_config()
     tp = TP.plan(cfg, args.world, args.moe_mode)
-    steps = {str(n): OP.plan_step(n, "tc", args.world).__dict__ | {"collective": OP.plan_step(n, "tc", args.world).collective.kind.value}
-             for n in (1, 5, 16, 64, 128, 1024)}
+    plans = {str(n): OP.plan_step(n, "tc", args.world, experts=cfg.n_routed_experts, top_k=cfg.top_k) for n in (1, 5, 16, 64, 128, 1024)}
+    steps = {n: p.__dict__ | {"collective": p.collective.kind.value} for n, p in plans.items()}
     print(json.dumps({"world": args.world, "moe_mode": args.moe_mode, "gb_per_rank": round(tp.bytes_per_rank() / 1e9, 2),
                       "heads_per_rank": tp.heads_per_rank, "inter_per_rank": tp.inter_per_rank, "vocab_per_rank": tp.vocab_per_rank,
                       "experts_per_rank": tp.experts_per_rank, "collectives_per_step": tp.collectives_per_step(), "tensors": tp.table(),

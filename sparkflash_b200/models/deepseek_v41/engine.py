@@ -667,10 +667,9 @@ class Engine:
     # sizes need two segments, the wider ones with a third more operand reads.
     GROUP_WIDER_PAIRS = 128
 
-    def _group_size(self, n: int, k: int, E_local: int) -> int:
-        if n < self.GROUP_WIDE_ROWS:
-            return 16
-        return 96 if n * k >= self.GROUP_WIDER_PAIRS * E_local and self.cfg.hidden_size % 256 == 0 else 64
+    def _group_size(self, n: int, k: int, E: int) -> int:
+        """Pairs per segment of a step of n rows that choose k of all the layer's E experts, wherever those are held."""
+        return _plan.expert_segment(n, k, E, self.cfg.hidden_size, self.GROUP_WIDE_ROWS, self.GROUP_WIDER_PAIRS)
 
     def _group_buffers(self, seg: int = 16):
         grp = self.__dict__.setdefault("_grp", {})
@@ -710,7 +709,7 @@ class Engine:
         cfg = self.cfg
         d = cfg.hidden_size
         E_local = self.w.experts_local or cfg.n_routed_experts
-        seg = self._group_size(n, k, E_local)
+        seg = self._group_size(n, k, cfg.n_routed_experts)
         g = self._group_buffers(seg)
         S = self._group_segments(n, k, E_local, seg)
         N.moe_plan(self.ids, self.wts, n, k, E_local, shared_here, S, g["seg_expert"], g["seg_count"], g["seg_weight"], g["seg_token"], g["pair_pos"],

@@ -192,7 +192,8 @@ class KernelResolver:
 MANY_ROWS = 128            # above: token-tiled GEMMs, bf16-GEMM coefficients, one-block-per-row fold
 TC_ATTENTION_ROWS = 64     # above: attention on tcgen05 (a tolerance arm)
 GROUP_MIN_ROWS = 4         # from here on the experts run grouped by expert
-GROUP_WIDE_ROWS = 100      # from here on segments hold up to 64 pairs (96 where experts have more: Engine._group_size)
+GROUP_WIDE_ROWS = 100      # from here on segments hold up to 64 pairs
+GROUP_WIDER_PAIRS = 128    # from this many pairs per expert on, 96
 HEAD_TC_MIN_ROWS = 1
 SELECT_LONG_ENTRIES = 32768   # rows longer than this (and few rows) use the chunked select
 
@@ -207,7 +208,7 @@ class StepPlan:
     wo_a: str                  # pair | pair_bulk | cuda_core
     coef: str                  # rows | gemm
     fold: str                  # cluster | rows
-    moe: str                   # token | seg16 | seg64 | cuda_core
+    moe: str                   # token | seg16 | seg64 | seg96 | cuda_core
     gate: str                  # gemv | gemm
     head: str                  # gemv | gemm
     index_scores: str          # cuda_core | tc
@@ -227,8 +228,16 @@ class StepPlan:
         return n
 
 
+def expert_segment(rows: int, top_k: int, experts: int, d: int, wide_rows: int = GROUP_WIDE_ROWS, wider_pairs: int = GROUP_WIDER_PAIRS) -> int:
+    """Pairs per segment of the grouped experts, of which there are ``experts`` in the layer (all ranks together: pairs of experts held elsewhere are
+    skipped, so the pairs an expert here can expect are those of the whole layer).  The wider down kernel takes two column tiles at a time."""
+    if rows < wide_rows:
+        return 16
+    return 96 if rows * top_k >= wider_pairs * experts and d % 256 == 0 else 64
+
+
 def plan_step(rows: int, arm: str = "tc", world: int = 1, d: int = 5120, head_dim: int = 512, collective_arm: str = "fused",
-              context_entries: int = 0) -> StepPlan:
+              context_entries: int = 0, experts: int = 384, top_k: int = 6) -> StepPlan:
     tc = arm == "tc"
     many = rows > MANY_ROWS
     return StepPlan(
@@ -238,7 +247,7 @@ def plan_step(rows: int, arm: str = "tc", world: int = 1, d: int = 5120, head_di
         wo_a=("pair_bulk" if rows > TC_ATTENTION_ROWS else "pair") if tc else "cuda_core",
         coef="gemm" if (tc and many) else "rows",
         fold="rows" if many else "cluster",
-        moe=("cuda_core" if not tc else "token" if rows < GROUP_MIN_ROWS else "seg64" if rows >= GROUP_WIDE_ROWS else "seg16"),
+        moe=("cuda_core" if not tc else "token" if rows < GROUP_MIN_ROWS else f"seg{expert_segment(rows, top_k, experts, d)}"),
         gate="gemm" if (tc and many) else "gemv",
         head="gemm" if (tc and HEAD_TC_MIN_ROWS <= rows <= 128) else "gemv",
         index_scores="tc" if tc else "cuda_core",

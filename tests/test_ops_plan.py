@@ -40,6 +40,41 @@ def test_step_plan_switches_variants_at_the_engine_thresholds():
     assert one.kernels_per_layer() < bulk.kernels_per_layer(index_layer=True, kv_source=True)
 
 
+@pytest.mark.parametrize("rows,experts,segment", [(99, 64, 16), (100, 64, 64), (1365, 64, 64), (1366, 64, 96), (1024, 384, 64), (4096, 384, 64), (8191, 384, 64),
+                                                  (8192, 384, 96)])
+def test_segments_follow_the_pairs_per_expert_of_the_whole_layer(monkeypatch, rows, experts, segment):
+    """The same sizes when one rank holds every expert and when eight hold an eighth each, and in the plan of the step."""
+    from types import SimpleNamespace
+    from sparkflash_b200.models.deepseek_v41 import engine as E
+    cfg = SimpleNamespace(hidden_size=5120, n_routed_experts=experts, top_k=6, swiglu_limit=10.0)
+    seen = []
+    names = SimpleNamespace(**{f: lambda *a, seg=None, **k: seen.append(seg) for f in ("moe_plan", "moe_permute", "umma_gate_up_grouped", "umma_down_grouped", "moe_combine")})
+    monkeypatch.setattr(E, "N", names)
+    mat = SimpleNamespace(tmap=None, atoms=None)
+
+    class Buffers(dict):
+        def __missing__(self, key):
+            return None
+
+    class Rank(E.Engine):
+        def __init__(self, local):
+            self.cfg, self.w, self.il, self.status, self.xq, self.xs, self.ids, self.wts = cfg, SimpleNamespace(experts_local=local), 2304, None, None, None, None, None
+            self.y_ffn = SimpleNamespace(stride=lambda i: 5120)
+
+        def _group_buffers(self, *a):
+            return Buffers(x_atom_bytes=0)
+
+        def _k(self):
+            pass
+    for local in (0, experts // 8):
+        seen.clear()
+        Rank(local)._ffn_grouped(rows, SimpleNamespace(w13=mat, s13=mat, w2=mat, s2=mat), 6, True)
+        assert set(seen) - {None} == {segment}, local
+    assert E.Engine.GROUP_WIDER_PAIRS == P.GROUP_WIDER_PAIRS
+    assert P.plan_step(rows, experts=experts).moe == f"seg{segment}"
+    assert P.plan_step(rows, experts=experts, d=5120 + 128).moe == f"seg{min(segment, 64)}"
+
+
 def test_collective_plan_forms_and_bytes():
     d = 5120
     assert P.plan_collective(8, d, 1).kind is P.CollectiveKind.NONE
