@@ -219,6 +219,9 @@ class Engine:
             self.tcb = TC.TcBuffers(self)
             self._splits = TC.pick_splits
             self._splits_bulk = TC.pick_splits_bulk
+            if any(T.w13 is not None for T in self.tcl):
+                for seg, rows in self._group_rows().items():      # now, and not inside the first step of each size
+                    self._group_buffers(seg, rows)
         elif arm != "cuda":
             raise ValueError(f"unknown arm {arm!r}")
         self.engram = engram          # engram.runtime.EngramRuntime or None
@@ -671,15 +674,24 @@ class Engine:
         """Pairs per segment of a step of n rows that choose k of all the layer's E experts, wherever those are held."""
         return _plan.expert_segment(n, k, E, self.cfg.hidden_size, self.GROUP_WIDE_ROWS, self.GROUP_WIDER_PAIRS)
 
-    def _group_buffers(self, seg: int = 16):
+    def _group_rows(self) -> dict[int, int]:
+        """Pairs per segment -> the most rows of a step that uses segments of that size."""
+        most = {}
+        for n in range(self.GROUP_MIN_ROWS, self.max_rows + 1):
+            most[self._group_size(n, self.cfg.top_k, self.cfg.n_routed_experts)] = n
+        return most
+
+    def _group_buffers(self, seg: int, n: int):
+        """Workspace of a step of n rows in segments of ``seg`` pairs, made with the engine for the most rows of a step that uses them.  Where the
+        rule has been changed since, a larger one takes its place; captured steps keep the one that they were captured with."""
         grp = self.__dict__.setdefault("_grp", {})
-        if seg not in grp:
+        if seg not in grp or grp[seg]["rows"] < n:
             from ... import codecs as CC
-            cfg, dev, R = self.cfg, self.dev, self.max_rows
+            cfg, dev, R = self.cfg, self.dev, max(n, self._group_rows().get(seg, 0))
             d, il = cfg.hidden_size, self.il
             S = self._group_segments(R, cfg.top_k, self.w.experts_local or cfg.n_routed_experts, seg)
             u8 = dict(dtype=torch.uint8, device=dev)
-            g = dict(S=S,
+            g = dict(rows=R, before=grp.get(seg),
                      seg_expert=torch.full((S,), -1, dtype=torch.int32, device=dev), seg_count=torch.zeros((S,), dtype=torch.int32, device=dev),
                      seg_weight=torch.zeros((S * seg,), dtype=torch.float32, device=dev), seg_token=torch.full((S * seg,), -1, dtype=torch.int32, device=dev),
                      pair_pos=torch.full((R * (cfg.top_k + 1),), -1, dtype=torch.int32, device=dev),
@@ -710,7 +722,7 @@ class Engine:
         d = cfg.hidden_size
         E_local = self.w.experts_local or cfg.n_routed_experts
         seg = self._group_size(n, k, cfg.n_routed_experts)
-        g = self._group_buffers(seg)
+        g = self._group_buffers(seg, n)
         S = self._group_segments(n, k, E_local, seg)
         N.moe_plan(self.ids, self.wts, n, k, E_local, shared_here, S, g["seg_expert"], g["seg_count"], g["seg_weight"], g["seg_token"], g["pair_pos"],
                    seg=seg); self._k()

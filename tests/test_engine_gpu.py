@@ -765,6 +765,21 @@ def test_moe_segments_of_96_pairs_give_the_bits_of_16_pair_segments(tiny, rows):
     assert torch.equal(*outs)
 
 
+def test_workspaces_of_the_experts_are_made_with_the_engine(tiny):
+    """Steps of four rows, of a hundred, and of 128 pairs per expert bring no workspace of their own."""
+    from sparkflash_b200.models.deepseek_v41 import engine as E
+    cfg, ck, w, orc, dw = tiny
+    rows = 128 * cfg.n_routed_experts // cfg.top_k
+    prompt = _prompt(cfg, rows, seed=31)
+    e = E.Engine(dw, max_lanes=2, max_context=1024, max_rows=rows, arm="tc", use_graphs=False)
+    made = {seg: g["ypair"].data_ptr() for seg, g in e._grp.items()}
+    assert set(made) == {16, 64, 96} and [g["rows"] for g in e._grp.values()] == [99, rows - 1, rows]
+    for n in (4, 99, 100, rows - 1, rows):
+        e.step(prompt[:n], [0] * n, list(range(n)))
+    e.check_status()
+    assert made == {seg: g["ypair"].data_ptr() for seg, g in e._grp.items()} and all(g["before"] is None for g in e._grp.values())
+
+
 def test_guard_bands_stay_intact_over_decode_and_chunk_steps_and_report_a_changed_band(tiny):
     """Every device buffer of a guarded engine sits between two 256-byte bands of a fixed pattern: steps of every kind leave
     them intact (no kernel writes outside its buffers), and a band changed from the host is reported with the allocation's

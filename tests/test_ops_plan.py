@@ -75,6 +75,48 @@ def test_segments_follow_the_pairs_per_expert_of_the_whole_layer(monkeypatch, ro
     assert P.plan_step(rows, experts=experts, d=5120 + 128).moe == f"seg{min(segment, 64)}"
 
 
+def test_workspaces_of_the_experts_cover_the_steps_that_use_them_and_no_more(monkeypatch):
+    """4,096 rows over 128 experts: segments of 16 pairs serve up to 99 rows, of 64 up to 2,730, of 96 the rest."""
+    from types import SimpleNamespace
+    from sparkflash_b200.models.deepseek_v41 import engine as E
+    nothing = lambda *a, **k: None
+    names = ("moe_plan", "moe_permute", "umma_gate_up_grouped", "umma_down_grouped", "moe_combine")
+    planned = []
+    monkeypatch.setattr(E, "N", SimpleNamespace(**dict.fromkeys(names, nothing), TensorMap=lambda *a: SimpleNamespace(ptr=0)))
+    E.N.moe_plan = lambda ids, wts, n, k, El, shared, S, expert, count, weight, token, pos, seg: planned.append(
+        expert.numel() >= S and token.numel() >= S * seg and pos.numel() >= n * (k + 1))
+    mat = SimpleNamespace(tmap=None, atoms=None)
+    T = SimpleNamespace(w13=mat, s13=mat, w2=mat, s2=mat)
+
+    class Stub(E.Engine):
+        def __init__(self):
+            self.cfg = SimpleNamespace(hidden_size=5120, n_routed_experts=128, top_k=6, swiglu_limit=10.0)
+            self.w, self.il, self.max_rows, self.dev = SimpleNamespace(experts_local=128), 2304, 4096, "meta"
+            self.status = self.xq = self.xs = self.ids = self.wts = None
+            self.y_ffn = SimpleNamespace(stride=lambda i: 5120)
+
+        def _k(self):
+            pass
+    eng = Stub()
+    for n in (4, 42, 43, 99, 100, 777, 2730, 2731, 4096):
+        eng._ffn_grouped(n, T, 6, True)
+    assert all(planned)
+    sets = {seg: sum(t.numel() * t.element_size() for t in g.values() if hasattr(t, "numel")) for seg, g in eng._grp.items()}
+    # a pair slot: its FP8 row, its FP8 activations, the 32-bit output, the scales, weight and token
+    slot = lambda seg: 5120 + 2304 + 4 * 5120 + 2 * (5120 + 2304) * (128 if seg <= 128 else seg) // seg // 32 + 64
+    assert set(sets) == {16, 64, 96}
+    assert sets[16] <= (128 + 99 * 6 // 16 + 7) * 16 * slot(16) and sets[64] <= (128 + 2730 * 6 // 64 + 43) * 64 * slot(64)
+    assert sets[96] <= (128 + 4096 * 6 // 96 + 43) * 96 * slot(96)
+    assert eng._group_rows() == {16: 99, 64: 2730, 96: 4096}
+    # a rule changed under a running engine: a larger workspace, the earlier one alive for what was captured with it
+    first = eng._grp[16]
+    eng.GROUP_WIDE_ROWS = 1000
+    eng._ffn_grouped(900, T, 6, True)
+    assert all(planned) and eng._grp[16]["rows"] == 999 and eng._grp[16]["before"] is first
+    eng._ffn_grouped(50, T, 6, True)
+    assert eng._grp[16]["before"] is first
+
+
 def test_collective_plan_forms_and_bytes():
     d = 5120
     assert P.plan_collective(8, d, 1).kind is P.CollectiveKind.NONE
