@@ -106,7 +106,6 @@ __global__ void __cluster_dims__(AT_SPLITS, 1, 1) __launch_bounds__(AT_THREADS, 
   const int n_sel = a.ckv_q ? a.sel_count[row] : 0;
   const int total = n_win + n_sel;
   const int e_lo = (int)((int64_t)total * sp / AT_SPLITS), e_hi = (int)((int64_t)total * (sp + 1) / AT_SPLITS);
-  const uint32_t M60 = bf16x2_splat(1.152921504606847e18f);      // 2^60
   float m_run = -1e30f, l_run = 0.f;                             // of head `warp`
   constexpr int DG = HD / 4;
   const int dg = tid % DG, hh4 = tid / DG;                       // values: dims 4 dg.., heads 4 hh4..
@@ -183,9 +182,9 @@ __global__ void __cluster_dims__(AT_SPLITS, 1, 1) __launch_bounds__(AT_THREADS, 
 #pragma unroll
         for (int j = 0; j < 4; ++j) o[j] = make_uint4(0u, 0u, 0u, 0u);
       } else if (base + el < n_win) {
-        const uint32_t m2 = bf16x2_splat(ue8m0_shifted((uint8_t)scl[i], 60));
-        fp8x16_to_bf16(raw0[i], M60, m2, o[0], o[1]);
-        fp8x16_to_bf16(raw1[i], M60, m2, o[2], o[3]);
+        const uint32_t m = ue8m0_splat((uint8_t)scl[i]);
+        fp8x16_to_bf16(raw0[i], m, o[0], o[1]);
+        fp8x16_to_bf16(raw1[i], m, o[2], o[3]);
       } else {
         uint32_t s0, s1;
         e4m3x2_splat((uint16_t)scl[i], s0, s1);

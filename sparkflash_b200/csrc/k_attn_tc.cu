@@ -335,7 +335,6 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(AttnTcArgs a) {
   uint32_t parity = 0;
   bool ok = true;
   const float sl2 = a.scale * LOG2E;
-  const uint32_t M60 = bf16x2_splat(1.152921504606847e18f);      // 2^60
 
   // the FP4 codes and scales of the NEXT tile's compressed entry are requested while the current tile is multiplied and
   // normalised, so that the gather's trip to L2 / HBM is not on the tile's critical path
@@ -360,10 +359,8 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(AttnTcArgs a) {
           for (int i = 0; i < 8; ++i) raw[i] = *reinterpret_cast<const uint4*>(kq + (b * 8 + i) * 16);
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            // block scale 2^(code - 127) times the 2^60 left over from the raw placement (2^-120 = 2^-60 2^-60)
-            const uint32_t m2 = bf16x2_splat(ue8m0_shifted(scb[(b * 8 + i) >> 1], 60));
             uint4 o0, o1;
-            fp8x16_to_bf16(raw[i], M60, m2, o0, o1);
+            fp8x16_to_bf16(raw[i], ue8m0_splat(scb[(b * 8 + i) >> 1]), o0, o1);
             const int c = half * 32 + (b * 8 + i) * 2;
             *reinterpret_cast<uint4*>(rowp + (c >> 3) * SLAB_BYTES + swz(key_slot, c & 7)) = o0;
             *reinterpret_cast<uint4*>(rowp + ((c + 1) >> 3) * SLAB_BYTES + swz(key_slot, (c + 1) & 7)) = o1;
@@ -726,7 +723,6 @@ __global__ void __launch_bounds__(THREADS64, 1) attn_tc64_kernel(AttnTcArgs a) {
   float m_run = -1e30f, l_run = 0.f;                                      // of this thread's head, the same in its eight threads
   bool ok = true;
   const float sl2 = a.scale * LOG2E;
-  const uint32_t M60 = bf16x2_splat(1.152921504606847e18f);      // 2^60
 
   // codes and scales of the NEXT tile's compressed entry are requested while the current tile is multiplied and normalised
   uint4 nraw[4];
@@ -755,10 +751,8 @@ __global__ void __launch_bounds__(THREADS64, 1) attn_tc64_kernel(AttnTcArgs a) {
         for (int i = 0; i < 8; ++i) raw[i] = *reinterpret_cast<const uint4*>(kq + i * 16);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          // block scale 2^(code - 127) times the 2^60 left over from the raw placement (2^-120 = 2^-60 2^-60)
-          const uint32_t m2 = bf16x2_splat(ue8m0_shifted((uint8_t)(sc >> (8 * (i >> 1))), 60));
           uint4 o0, o1;
-          fp8x16_to_bf16(raw[i], M60, m2, o0, o1);
+          fp8x16_to_bf16(raw[i], ue8m0_splat((uint8_t)(sc >> (8 * (i >> 1)))), o0, o1);
           *reinterpret_cast<uint4*>(rowp + (i >> 2) * SLAB_BYTES + swz(key_slot, (2 * i) & 7)) = o0;
           *reinterpret_cast<uint4*>(rowp + (i >> 2) * SLAB_BYTES + swz(key_slot, (2 * i + 1) & 7)) = o1;
         }

@@ -6,9 +6,10 @@ namespace sfb {
 
 // ---- cache codes -> bf16 by bit placement ----------------------------------------------------------------------
 // An E4M3 byte shifted into a bf16 (sign to bit 15, the seven exponent|mantissa bits to bits 4..10) is the code's value
-// times 2^-120, subnormal codes included (they land on bf16 subnormals).  Two exact bf16 multiplications by powers of two (the
-// second one carrying the block scale) undo the factor.  An E2M1 nibble is looked up and multiplied by its E4M3 scale: two significant
-// bits times four.  Every intermediate is representable, so the result is the exact product.
+// times 2^-120, subnormal codes included (they land on bf16 subnormals).  Two exact bf16 multiplications by powers of two, 2^120 and
+// the block scale, make it the entry: first the code's value, then the product, so that any scale gives what the entry is - beyond
+// bf16's range an infinity.  An E2M1 nibble is looked up and multiplied by its E4M3 scale: two significant bits times four.  Every
+// intermediate is representable, so the result is the exact product.
 __device__ __forceinline__ uint32_t e4m3x2_to_bf16x2_raw(uint32_t two_bytes_in_high_halves) {
   // input: byte a in bits 8..15, byte b in bits 24..31
   const uint32_t t = two_bytes_in_high_halves;
@@ -22,16 +23,19 @@ __device__ __forceinline__ uint32_t bf16x2_splat(float f) {
   __nv_bfloat162 r = __float2bfloat162_rn(f);
   return *reinterpret_cast<uint32_t*>(&r);
 }
-// 16 E4M3 codes (one uint4) with one power-of-two scale -> two uint4 of bf16; m1, m2: splatted bf16 multipliers
-__device__ __forceinline__ void fp8x16_to_bf16(const uint4& v, uint32_t m1, uint32_t m2, uint4& o0, uint4& o1) {
+// a UE8M0 scale, 2^(code - 127), in both halves of a word: the code is the exponent field, and 0 is a subnormal
+__device__ __forceinline__ uint32_t ue8m0_splat(uint8_t code) { return code ? (uint32_t)code * 0x00800080u : 0x00400040u; }
+// 16 E4M3 codes (one uint4) with one splatted power-of-two scale -> two uint4 of bf16
+__device__ __forceinline__ void fp8x16_to_bf16(const uint4& v, uint32_t scale, uint4& o0, uint4& o1) {
+  constexpr uint32_t M120 = 0x7b807b80u;      // 2^120, twice
   const uint32_t w[4] = {v.x, v.y, v.z, v.w};
   uint32_t r[8];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const uint32_t lo = __byte_perm(w[i], 0u, 0x1404);   // bytes: [0, b0, 0, b1] -> b0 in bits 8..15, b1 in bits 24..31
     const uint32_t hi = __byte_perm(w[i], 0u, 0x3424);   // b2, b3
-    r[2 * i] = bf16x2_mul(bf16x2_mul(e4m3x2_to_bf16x2_raw(lo), m1), m2);
-    r[2 * i + 1] = bf16x2_mul(bf16x2_mul(e4m3x2_to_bf16x2_raw(hi), m1), m2);
+    r[2 * i] = bf16x2_mul(bf16x2_mul(e4m3x2_to_bf16x2_raw(lo), M120), scale);
+    r[2 * i + 1] = bf16x2_mul(bf16x2_mul(e4m3x2_to_bf16x2_raw(hi), M120), scale);
   }
   o0 = make_uint4(r[0], r[1], r[2], r[3]);
   o1 = make_uint4(r[4], r[5], r[6], r[7]);

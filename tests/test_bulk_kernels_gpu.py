@@ -259,6 +259,37 @@ def test_attention_of_64_heads_at_the_edges_of_key_tiles(selected):
     assert (a.float() - b.float()).abs().max() <= 2 ** -6 * a.float().abs().max()
 
 
+@pytest.mark.parametrize("kernel", ["rows", "tc"])
+@pytest.mark.parametrize("heads", [16, 32, 64])
+def test_attention_takes_window_entries_of_any_scale(kernel, heads):
+    """Entries 2^80 times as large under queries 2^80 times as small have the same scores, and outputs 2^80 times as large: powers of two change no
+    bit of a significand.  An entry whose scale is infinite leaves nothing finite."""
+    from sparkflash_b200.ops import native as N
+    dev = "cuda"
+    c = _attention_case(heads, [300, 899, 17], False, seed=9)
+    n, hd, rd = c["n"], c["hd"], c["rd"]
+    rope = torch.zeros(n, 1, rd // 2, 2, dtype=torch.float32, device=dev)
+    N.rope_table([c["invf"].to(dev)], [1], c["pos"].to(dev), rope, n)
+    status = torch.zeros(4, dtype=torch.int32, device=dev)
+
+    def run(q, ws):
+        out = torch.zeros(n, heads * hd, dtype=torch.bfloat16, device=dev)
+        args = (q.to(dev), heads * hd, rope[:, 0], c["lane"].to(dev), c["pos"].to(dev), c["wq"].to(dev), ws.to(dev), None, None, None, None, c["K"],
+                c["sink"].to(dev), out, n, heads, hd, rd, c["window"], c["ring"], hd ** -0.5)
+        N.attn_rows(*args) if kernel == "rows" else N.attn_tc(*args, status=status)
+        return out.cpu()
+    plain = run(c["q"], c["ws"])
+    assert int(c["ws"].max()) + 80 < 240
+    large = run((c["q"].double() * 2.0 ** -80).to(torch.bfloat16), c["ws"] + 80)
+    assert torch.equal(large.double(), plain.double() * 2.0 ** 80)
+    ws = c["ws"].clone()
+    ws[0, 17] = ws[1, 899 % c["ring"]] = 255
+    assert c["lane"].tolist() == [0, 1, 0]
+    bad = run(c["q"], ws).isfinite().view(n, -1)
+    assert bad[0].all() and not bad[1].any() and not bad[2].any()
+    assert status.tolist()[0] == 0
+
+
 @pytest.mark.parametrize("n,k,E,seg", [(1, 6, 64, 16), (42, 6, 64, 16), (43, 6, 64, 16), (100, 6, 64, 64), (777, 6, 5, 64), (1000, 2, 300, 96), (3, 1, 1, 16)])
 def test_expert_plan_gives_every_pair_a_place(n, k, E, seg):
     """Up to 256 pairs by one block in pair order, more by a cluster; experts that are not here (-1), unused experts, the shared expert's rows."""
