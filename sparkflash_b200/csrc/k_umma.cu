@@ -1063,15 +1063,20 @@ umma_pair_persistent_kernel(const __grid_constant__ CUtensorMap tmapA, const __g
       const uint32_t idesc = make_idesc(0, 0, 128, 128);
       uint32_t it = 0;
       int lt = 0;
+      long long c_acc = 0, c_full = 0, c_all0 = SFB_MARKS_ON ? clock64() : 0;      // cycles waiting for a free accumulator set / for data
       for (int t = blockIdx.x; t < total && !S.fail; t += gridDim.x, ++lt) {
         const int buf = lt & 1;
+        const long long w0 = SFB_MARKS_ON ? clock64() : 0;
         if (lt >= 2 && !mbar_wait(&S.acc_empty[buf], ((lt >> 1) - 1) & 1)) { S.fail = 3; break; }
+        if (SFB_MARKS_ON) c_acc += clock64() - w0;
         tc_fence_after();
         const uint32_t t_acc = tmem + (uint32_t)buf * 128;
         bool ok = true;
         for (int i = 0; i < ksteps; ++i, ++it) {
           const int s = it % ST;
+          const long long w1 = SFB_MARKS_ON ? clock64() : 0;
           if (!mbar_wait(&S.full[s], (it / ST) & 1)) { S.fail = 2; ok = false; break; }
+          if (SFB_MARKS_ON) c_full += clock64() - w1;
           tc_fence_after();
           const uint32_t sf_slot = (it & 1u) * 4;
           tc_cp_sf(t_sfa + sf_slot, make_desc(smem_u32(S.sfa[s]), 128, 0, 0));
@@ -1088,16 +1093,26 @@ umma_pair_persistent_kernel(const __grid_constant__ CUtensorMap tmapA, const __g
         tc_commit(&S.acc_full[buf]);      // arrives even after a failed wait, so the epilogue never waits for its limit
         if (!ok) break;
       }
+      if (SFB_MARKS_ON && a.marks && (int)blockIdx.x < a.marks_cap) {      // per CTA: tiles, total, waiting-for-set, waiting-for-data cycles
+        a.marks[(size_t)blockIdx.x * 16 + 0] = (unsigned long long)lt;
+        a.marks[(size_t)blockIdx.x * 16 + 1] = (unsigned long long)(clock64() - c_all0);
+        a.marks[(size_t)blockIdx.x * 16 + 2] = (unsigned long long)c_acc;
+        a.marks[(size_t)blockIdx.x * 16 + 3] = (unsigned long long)c_full;
+      }
     }
   } else {
     const int q = warp & 3, tid = q * 32 + lane;
     bool pending = false;      // this thread has bulk copies of the previous tile in flight
     int lt = 0;
+    long long c_wait = 0;      // cycles the epilogue waited for an accumulator (marks builds)
+    const long long c_ep0 = SFB_MARKS_ON ? clock64() : 0;
     for (int t = blockIdx.x; t < total; t += gridDim.x, ++lt) {
       const int buf = lt & 1, wt = t % n_all, tt = t / n_all;
       if (warp == 2) {
         bool got = true;
+        const long long w2 = SFB_MARKS_ON ? clock64() : 0;
         if (lane == 0) got = mbar_wait(&S.acc_full[buf], (lt >> 1) & 1) && !S.fail;
+        if (SFB_MARKS_ON && lane == 0) c_wait += clock64() - w2;
         got = __shfl_sync(0xffffffffu, got ? 1 : 0, 0) != 0;
         if (lane == 0 && !got) S.ep_ok = 0;
       }
@@ -1172,6 +1187,10 @@ umma_pair_persistent_kernel(const __grid_constant__ CUtensorMap tmapA, const __g
       }
     }
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");      // every copy of this thread has been written
+    if (SFB_MARKS_ON && a.marks && warp == 2 && lane == 0 && (int)blockIdx.x < a.marks_cap) {
+      a.marks[(size_t)blockIdx.x * 16 + 4] = (unsigned long long)(clock64() - c_ep0);
+      a.marks[(size_t)blockIdx.x * 16 + 5] = (unsigned long long)c_wait;
+    }
     if ((S.fail || !S.ep_ok) && lane == 0 && q == 0) status_set(a.status, ST_TIMEOUT, 100 + S.fail, blockIdx.x, lt);
   }
   tc_fence_before();
@@ -2281,7 +2300,9 @@ static thread_local GatherSpec g_gather;
 
 // Tuning switches for measurements (0 = the shipped choice): [1] stages of the 64-pair down projection (2 shipped; 3, 4),
 // [2] stages of the 64-pair gate/up (2 = two CTAs per SM; 3, 5 = one CTA per SM), [3] / [4] segment-major grid order of the
-// grouped down / gate-up kernels, [5] persistent many-row dense kernel, [6] persistent 64-pair gate/up kernel, [7] persistent 64-pair down kernel (1 = never, 2 = whenever the shape allows, 3 = the same with one column tile per work item).
+// grouped down / gate-up kernels, [5] persistent many-row dense kernels, of one term and of two, [6] persistent 64-pair gate/up kernel, [7] persistent
+// 64-pair down kernel (1 = never, 2 = whenever the shape allows, 3 = the same with one column tile per work item).  Segments of 96 pairs have the persistent
+// kernels alone, whatever [6] and [7] say: Engine.GROUP_WIDER_PAIRS chooses between them and segments of 64.
 static int g_tune[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 // Phase marks (um_mark) of the NEXT launch of a tensor-core GEMM of this library: cleared by that launch.
 static thread_local unsigned long long* g_marks = nullptr;
@@ -2466,10 +2487,11 @@ int sfb_umma_pair_bulk(const void* tmapA, const void* tmapB, const void* sfa, in
   a.out_q = (uint8_t*)out_q; a.out_q_atom = (uint8_t*)out_q_atom; a.status = (Status*)status;
   a.force_bulk = 1;
   a.tok_tiles = (n_rows + 63) / 64;
-  // two rounds of tiles and more, whole output rows as bulk copies: one persistent CTA per SM
+  // Two rounds of tiles and more, whole output rows as bulk copies: one persistent CTA per SM (g_tune[5]: 1 = never, 2 = whenever the shape allows).  At
+  // 296 to 4,096 tiles it takes 0.63 to 0.88 of the time of the CTAs of one tile each (304 tiles 37 us against 53, 4,096 tiles 250 against 369).
   const long long tiles = (long long)(N / 128) * groups * a.tok_tiles;
   if (splits == 1 && out_b && !out_f && out_stride % 128 == 0 && (uintptr_t)out_b % 16 == 0 && (uintptr_t)out_q % 16 == 0 && (uintptr_t)out_q_atom % 4 == 0 &&
-      tiles >= 296 && tiles < (1ll << 31) && g_push.n == 0 && g_gather.n == 0) {
+      g_tune[5] != 1 && (g_tune[5] == 2 || tiles >= 296) && tiles < (1ll << 31) && g_push.n == 0 && g_gather.n == 0) {
     const size_t smem = sizeof(UmmaPairPersistSmem) + 1024;
     static bool done = false;
     if (!done) { cudaFuncSetAttribute(umma_pair_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); done = true; }

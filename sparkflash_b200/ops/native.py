@@ -432,7 +432,7 @@ def bf16_map(t: torch.Tensor, rows: int, K: int, box_rows: int) -> TensorMap:
 
 
 def umma_tune(key: int, value: int) -> None:
-    """Measurement switch of the MoE launchers (csrc/k_umma.cu g_tune); 0 restores the shipped choice."""
+    """Measurement switch of the MoE and many-row launchers (csrc/k_umma.cu g_tune); 0 restores the shipped choice."""
     _check(lib().sfb_umma_tune(c_int(key), c_int(value)), "umma_tune")
 
 

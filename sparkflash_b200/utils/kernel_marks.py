@@ -68,14 +68,15 @@ def summarize_attention(buf: torch.Tensor) -> dict:
 
 
 def summarize_persistent(buf: torch.Tensor, kind: str) -> dict:
-    """Cycle counters of the persistent MoE kernels (one record per CTA).  ``gate_up``: tiles, MMA thread total / waiting for a
-    free accumulator set / waiting for data, epilogue total / waiting for an accumulator.  ``down``: the same three of the MMA
+    """Cycle counters of the persistent kernels (one record per CTA).  ``gate_up`` and ``pair`` (the two-term projection): tiles, MMA thread total / waiting for
+    a free accumulator set / waiting for data, epilogue total / waiting for an accumulator.  ``down``: the same three of the MMA
     thread, the scale-copy thread's total / waiting for a stage, k-steps, the producer's total / waiting for a free stage."""
     m = buf.detach().cpu().view(-1, 16).double()
     m = m[m[:, 0] > 0]
     if not m.shape[0]:
         return {"ctas": 0}
-    names = {"gate_up": ("tiles", "mma_cycles", "mma_wait_set", "mma_wait_data", "epilogue_cycles", "epilogue_wait_acc"),
+    gemm = ("tiles", "mma_cycles", "mma_wait_set", "mma_wait_data", "epilogue_cycles", "epilogue_wait_acc")
+    names = {"gate_up": gemm, "pair": gemm,
              "down": ("tiles", "mma_cycles", "mma_wait_set", "mma_wait_scales", "copier_cycles", "copier_wait_stage", "ksteps",
                       "producer_cycles", "producer_wait_free")}[kind]
     return {"ctas": int(m.shape[0]), **{n: round(float(m[:, i].mean()), 1) for i, n in enumerate(names)}}

@@ -21,9 +21,10 @@ def main() -> None:
     ap.add_argument("--experts", type=int, default=128)
     ap.add_argument("--layers", type=int, default=3)
     ap.add_argument("--steps", type=int, default=12, help="prompt chunks to run (the last one is the profiled / timed one)")
-    ap.add_argument("--persistent-counters", action="store_true", help="read moe_gate_up / moe_down marks as the persistent kernels' cycle counters")
+    ap.add_argument("--persistent-counters", action="store_true", help="read moe_gate_up / moe_down / wo_a marks as the persistent kernels' cycle counters")
     ap.add_argument("--marks", default="", help="kernels whose in-kernel phase marks are printed for the last step, e.g. moe_down,moe_gate_up")
-    ap.add_argument("--tune", default="", help="measurement switches of the MoE launchers, key=value[,key=value]")
+    ap.add_argument("--tune", default="", help="measurement switches of the MoE and many-row launchers, key=value[,key=value]")
+    ap.add_argument("--wider-pairs", type=int, default=None, help="pairs per expert from which segments hold 96 (Engine.GROUP_WIDER_PAIRS)")
     args = ap.parse_args()
     from sparkflash_b200.config import reduced_config
     from sparkflash_b200.models.deepseek_v41 import engine as E, prepare as P
@@ -37,6 +38,8 @@ def main() -> None:
     ctx = max(2048, rows * args.steps + 64)
     eng = E.Engine(w, max_lanes=max(2, rows if args.decode else 2), max_context=ctx, max_rows=max(64, rows), arm="tc",
                    synthetic_scales=True, use_graphs=False)
+    if args.wider_pairs is not None:
+        eng.GROUP_WIDER_PAIRS = args.wider_pairs
     prompt = torch.randint(0, cfg.vocab_size, (ctx,)).tolist()
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     if args.decode:
@@ -67,8 +70,8 @@ def main() -> None:
         elif name == "seam":
             words = N.seam_read_marks(rows)
             print(name, KM.summarize_seam(words, rows) if words is not None else "no marks in this library")
-        elif name in ("moe_gate_up", "moe_down") and args.persistent_counters:
-            print(name, KM.summarize_persistent(buf, "gate_up" if name == "moe_gate_up" else "down"))
+        elif name in ("moe_gate_up", "moe_down", "wo_a") and args.persistent_counters:
+            print(name, KM.summarize_persistent(buf, {"moe_gate_up": "gate_up", "moe_down": "down", "wo_a": "pair"}[name]))
         else:
             print(name, KM.summarize(buf))
     if not args.decode:

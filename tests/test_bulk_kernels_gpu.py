@@ -132,6 +132,36 @@ def test_persistent_pair_gemm_gives_the_bits_of_the_tiles(n):
     assert status.tolist()[0] == 0
 
 
+@pytest.mark.parametrize("n", [1, 64, 65, 129])
+def test_pair_gemm_gives_the_same_bits_under_either_switch(n):
+    """The measurement switch of the many-row kernels: one CTA per tile, or the persistent kernel below its rule, with fewer tiles than SMs."""
+    from sparkflash_b200.ops import native as N
+    dev, groups, N_, K = "cuda", 2, 384, 896
+    g = torch.Generator().manual_seed(n)
+    q, s = C.weight_quant_fp8_block32(torch.randn(groups * N_, K, generator=g) * 0.05)
+    nblk, KB, KBo = (n + 63) // 64, groups * K // 32, groups * N_ // 32
+    x = torch.randn(n, groups * K, generator=g).to(torch.bfloat16).to(dev)
+    xq, block = torch.zeros(nblk * 128, groups * K, dtype=torch.uint8, device=dev), C.sf_bytes(128, KB)
+    atom = torch.full((nblk * block,), 127, dtype=torch.uint8, device=dev)
+    for b in range(nblk):
+        N.quant_rows(x[64 * b:], xq[128 * b:], None, atom[b * block:], min(64, n - 64 * b), groups * K, split=True, split_off=64)
+    ta, tb = N.TensorMap(q.to(dev).contiguous(), groups * N_, K, K, 128), N.TensorMap(xq, nblk * 128, groups * K, groups * K, 128)
+    sfa = C.scales_to_prepared(s, groups * N_, 32).to(dev)
+    scratch, tickets = torch.zeros(64 * 128 * 128, device=dev), torch.zeros(64, dtype=torch.int32, device=dev)
+    status, outs = torch.zeros(4, dtype=torch.int32, device=dev), []
+    try:
+        for arm in (1, 2):
+            N.umma_tune(5, arm)
+            out = torch.full((n, groups * N_), 9.0, dtype=torch.bfloat16, device=dev)
+            oq = torch.zeros(n, groups * N_, dtype=torch.uint8, device=dev)
+            oa = torch.full((C.sf_bytes(n, KBo),), 127, dtype=torch.uint8, device=dev)
+            N.umma_pair_bulk(ta, tb, sfa, atom, n, N_, K, groups=groups, scratch=scratch, tickets=tickets, out_b=out, out_q=oq, out_q_atom=oa, status=status)
+            outs.append((out.cpu(), oq.cpu(), C.prepared_to_scales(oa.cpu(), n, KBo)))
+    finally:
+        N.umma_tune(5, 0)
+    assert all(torch.equal(*p) for p in zip(*outs)) and status.tolist()[0] == 0
+
+
 def _attention_case(heads, rows, with_compressed, seed):
     from sparkflash_b200.models.deepseek_v41 import oracle as O
     from sparkflash_b200.config import full_config

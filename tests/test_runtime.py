@@ -133,6 +133,7 @@ def test_mark_summaries_of_the_attention_seam_and_persistent_kernels():
     pv[1, :9] = torch.tensor([22, 1200, 70, 500, 1100, 800, 396, 1180, 620])
     down = KM.summarize_persistent(pc, "down")
     assert down["ctas"] == 2 and down["tiles"] == 21.0 and down["mma_wait_scales"] == 400.0 and down["producer_wait_free"] == 520.0
+    assert KM.summarize_persistent(pc, "pair") == KM.summarize_persistent(pc, "gate_up") != down
     gu = KM.summarize_persistent(pc, "gate_up")
     assert gu["mma_wait_data"] == 400.0 and "ksteps" not in gu
 
