@@ -320,6 +320,89 @@ def test_attention_takes_window_entries_of_any_scale(kernel, heads):
     assert status.tolist()[0] == 0
 
 
+def test_attention_of_64_heads_gives_the_bits_of_two_groups_of_32():
+    """attn_tc64_kernel against attn_tc_kernel<32>: bf16 rows, both FP8 terms and their scales, over rows whose tiles end at, before and after 128 keys and
+    whose running maximum jumps; without the bf16 rows the FP8 terms are the same."""
+    from sparkflash_b200.ops import native as N
+    dev, heads, half = "cuda", 64, 32
+    rows = [0, 5, 126, 127, 128, 129, 255, 300, 383, 384, 640, 899] + list(range(700, 756))
+    c = _attention_case(heads, rows, True, seed=13)
+    n, hd, rd = c["n"], c["hd"], c["rd"]
+    for r in range(n):      # selected entries between none and all of them
+        c["cnt"][r] = min(int(c["cnt"][r]), [0, 1, 127, 128, 129, 512][r % 6])
+        c["sel"][r, int(c["cnt"][r]):] = -1
+    c["q"][1::3] *= 8
+    assert c["K"] == 512 and n > 64
+    rope = torch.zeros(n, 1, rd // 2, 2, dtype=torch.float32, device=dev)
+    N.rope_table([c["invf"].to(dev)], [1], c["pos"].to(dev), rope, n)
+    q, nblk = c["q"].to(dev), (n + 63) // 64
+    status = torch.zeros(4, dtype=torch.int32, device=dev)
+    caches = [t.to(dev) for t in (c["lane"], c["pos"], c["wq"], c["ws"], C.pack_nibbles(c["cq"]), c["cs"], c["sel"], c["cnt"])]
+
+    def run(first, m, rows_out=True):
+        out = torch.zeros(n, m * hd, dtype=torch.bfloat16, device=dev)
+        oq = torch.zeros(nblk * 128, m * hd, dtype=torch.uint8, device=dev)
+        atom = torch.full((C.sf_bytes(nblk * 128, m * hd // 32),), 127, dtype=torch.uint8, device=dev)
+        N.attn_tc(q[:, first * hd:], heads * hd, rope[:, 0], *caches, c["K"], c["sink"][first:first + m].to(dev), out if rows_out else None, n, m, hd, rd,
+                  c["window"], c["ring"], hd ** -0.5, out_q=oq, out_atom=atom, pair_block=64, status=status)
+        return out.cpu(), oq.cpu(), C.prepared_to_scales(atom.cpu(), nblk * 128, m * hd // 32)
+    whole = run(0, heads)
+    halves = [torch.cat(p, 1) for p in zip(run(0, half), run(half, half))]
+    assert all(torch.equal(a, b) for a, b in zip(whole, halves)) and whole[0].float().abs().sum() > 0
+    for m in (half, heads):
+        kept, bare = run(0, m), run(0, m, rows_out=False)
+        assert torch.equal(kept[1], bare[1]) and torch.equal(kept[2], bare[2]) and not bare[0].any()
+    assert status.tolist()[0] == 0
+
+
+@pytest.mark.parametrize("d,inter,counts", [(1024, 384, (95, 96, 97, 200, 0, 1, 33, 288)), (1280, 128, (191, 192, 193, 64, 63, 0, 500))])
+def test_expert_segments_of_any_size_give_the_same_bits(d, inter, counts):
+    """Gate/up, activation and down over segments of 16, 64 and 96 pairs, for experts with a pair less and more than whole segments, with several segments
+    and with none, and the shared expert: more than three work items per SM, so that both accumulator sets, the ring of stages and the staging
+    buffers are used again and again."""
+    from sparkflash_b200.ops import native as N
+    dev, E, k = "cuda", 32 * len(counts), 2
+    g = torch.Generator().manual_seed(d)
+    ids = torch.cat([torch.full((counts[e % len(counts)],), e) for e in range(E)])
+    if ids.numel() % k:
+        ids = torch.cat([ids, torch.tensor([-1])])
+    ids = ids[torch.randperm(ids.numel(), generator=g)].int().view(-1, k).to(dev)
+    n = ids.shape[0]
+    wts = torch.rand(n, k, generator=g).to(dev)
+    xq, xs = C.act_quant_fp8(torch.randn(n, d, generator=g))
+    xq, xs = xq.to(dev), xs.to(dev)
+    byte = lambda lo, hi, *shape: torch.randint(lo, hi, shape, generator=g, dtype=torch.uint8).to(dev)
+    w13, w2, s13, s2 = byte(0, 256, E * 2 * inter, d // 2), byte(0, 256, E * d, inter // 2), byte(0, 120, 2 * inter, d), byte(0, 120, d, inter)
+    maps = [N.TensorMap(w13, E * 2 * inter, d, d // 2, 128, fp4=True), N.TensorMap(s13, 2 * inter, d, d, 128),
+            N.TensorMap(w2, E * d, inter, inter // 2, 128, fp4=True), N.TensorMap(s2, d, inter, inter, 128)]
+    atoms = [byte(117, 121, C.sf_bytes(r, kk // 32)) for r, kk in ((E * 2 * inter, d), (2 * inter, d), (E * d, inter), (d, inter))]
+    status, outs = torch.zeros(4, dtype=torch.int32, device=dev), []
+    for seg in (16, 64, 96):
+        S = min(n * k, E + n * k // seg) + -(-n // seg)
+        i32 = lambda m: torch.full((m,), -1, dtype=torch.int32, device=dev)
+        expert, count, token, pos, weight = i32(S), i32(S), i32(S * seg), i32(n * (k + 1)), torch.zeros(S * seg, device=dev)
+        N.moe_plan(ids, wts, n, k, E, True, S, expert, count, weight, token, pos, seg=seg)
+        xp, act = torch.zeros(S * seg, d, dtype=torch.uint8, device=dev), torch.zeros(S * seg, inter, dtype=torch.uint8, device=dev)
+        xa = torch.full((S, C.sf_bytes(seg, d // 32)), 127, dtype=torch.uint8, device=dev)
+        aa = torch.full((S, C.sf_bytes(seg, inter // 32)), 127, dtype=torch.uint8, device=dev)
+        y = torch.zeros(S * seg, d, device=dev)
+        N.moe_permute(xq, xs, token, xp, xa, S * seg, d, C.sf_bytes(seg, d // 32), seg=seg)
+        N.umma_gate_up_grouped(maps[0], maps[1], N.TensorMap(xp, S * seg, d, d, seg), atoms[0], atoms[1], xa, expert, count, weight, act, aa, S, d, inter, 10.0,
+                               status=status, seg=seg)
+        N.umma_down_grouped(maps[2], maps[3], N.TensorMap(act, S * seg, inter, inter, seg), atoms[2], atoms[3], aa, expert, count, y, S, d, inter,
+                            status=status, seg=seg)
+        pos = pos.view(n, k + 1).long()
+        if seg == 96:
+            items = int((expert != -1).sum()) * min(inter // 128, d // 256)
+            assert items > 3 * torch.cuda.get_device_properties(0).multi_processor_count and int((count == 96).sum()) > E // len(counts)
+        outs.append((pos >= 0, act[pos.clamp(min=0)], y[pos.clamp(min=0)]))
+    here = outs[0][0]
+    assert status.tolist()[0] == 0 and torch.equal(here[:, :k], ids >= 0) and here[:, k].all()
+    for other in outs[1:]:
+        assert all(torch.equal(a[here], b[here]) for a, b in zip(outs[0], other))
+    assert outs[0][2][here].isfinite().all() and outs[0][2][here].abs().amax(1).min() > 0
+
+
 @pytest.mark.parametrize("n,k,E,seg", [(1, 6, 64, 16), (42, 6, 64, 16), (43, 6, 64, 16), (100, 6, 64, 64), (777, 6, 5, 64), (1000, 2, 300, 96), (3, 1, 1, 16)])
 def test_expert_plan_gives_every_pair_a_place(n, k, E, seg):
     """Up to 256 pairs by one block in pair order, more by a cluster; experts that are not here (-1), unused experts, the shared expert's rows."""
