@@ -676,10 +676,9 @@ class Engine:
 
     def _group_rows(self) -> dict[int, int]:
         """Pairs per segment -> the most rows of a step that uses segments of that size."""
-        most = {}
-        for n in range(self.GROUP_MIN_ROWS, self.max_rows + 1):
-            most[self._group_size(n, self.cfg.top_k, self.cfg.n_routed_experts)] = n
-        return most
+        k, E, R = self.cfg.top_k, self.cfg.n_routed_experts, self.max_rows
+        last = sorted({min(R, self.GROUP_WIDE_ROWS - 1), min(R, -(-self.GROUP_WIDER_PAIRS * E // k) - 1), R})      # before each line of the rule
+        return {self._group_size(n, k, E): n for n in last if n >= self.GROUP_MIN_ROWS}
 
     def _group_buffers(self, seg: int, n: int):
         """Workspace of a step of n rows in segments of ``seg`` pairs, made with the engine for the most rows of a step that uses them.  Where the

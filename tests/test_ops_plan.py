@@ -108,6 +108,9 @@ def test_workspaces_of_the_experts_cover_the_steps_that_use_them_and_no_more(mon
     assert sets[16] <= (128 + 99 * 6 // 16 + 7) * 16 * slot(16) and sets[64] <= (128 + 2730 * 6 // 64 + 43) * 64 * slot(64)
     assert sets[96] <= (128 + 4096 * 6 // 96 + 43) * 96 * slot(96)
     assert eng._group_rows() == {16: 99, 64: 2730, 96: 4096}
+    for eng.max_rows in (3, 4, 98, 99, 100, 101, 2730, 2731, 2732):
+        assert eng._group_rows() == {eng._group_size(n, 6, 128): n for n in range(4, eng.max_rows + 1)}
+    eng.max_rows = 4096
     # a rule changed under a running engine: a larger workspace, the earlier one alive for what was captured with it
     first = eng._grp[16]
     eng.GROUP_WIDE_ROWS = 1000
