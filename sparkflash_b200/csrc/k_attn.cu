@@ -77,8 +77,9 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; a
 // The partial (max, sum, accumulator) of every head stays in shared memory, and after a cluster barrier CTA rank h merges head h across the eight
 // CTAs in rank order through distributed shared memory - no global scratch, no atomics.  The split is a function of the row alone, so a
 // row's bits do not depend on the batch.
-// One row is bound by latency (ids, then codes; barriers; the merge), sixteen by the issue of the products.  640 entries, 64 heads, rows 4 / 16 / 64: 25 / 93 / 334 us; with four
-// heads per CTA, eight entries at a time decoded to fp32 and a warp per head: 45 / 169 / 616.
+// One row is bound by latency (ids, then codes; barriers; the merge), sixteen by the issue of the products.  640 entries, 64 heads, rows 4 / 16 / 64:
+// 25 / 93 / 334 us.  A rank with fewer heads has fewer CTAs and is no worse off than with four heads in each: L2 flushed, 1 / 16 / 64 rows, eight heads 23 / 31 / 57 us
+// against 47 / 49 / 107, sixteen 23 / 33 / 104 against 45 / 55 / 199, four 23 / 31 / 56 against 45 / 49 / 59.
 template <int HD>
 __global__ void __cluster_dims__(AT_SPLITS, 1, 1) __launch_bounds__(AT_THREADS, 2) attn_rows_kernel(AttnArgs a) {
   constexpr int EPL = HD / 32;          // elements per share

@@ -14,7 +14,7 @@
 // fp32: this kernel is a tolerance arm, not a bit-exact one).  Softmax is online over tiles of 128 keys: the
 // score tile goes TMEM -> registers -> shared memory (transposed), threads then own heads, and the running
 // accumulator in TMEM is rescaled per column when a head's maximum moves.  More than 32 heads: attn_tc64_kernel below, the same
-// arithmetic laid out for 64 heads per CTA.  The sink enters the denominator only.
+// arithmetic laid out for 64 heads per CTA, with the bits of the 32-head form.  The sink enters the denominator only.
 // Query RoPE on load, inverse RoPE on the output's rope slice, optional two-term FP8 copy for the wo_a GEMM.
 //
 // No cluster, no multicast; every mbarrier wait is bounded and reports through the status word.
@@ -657,8 +657,8 @@ struct AttnTc64Smem {
 };
 constexpr int THREADS64 = 512;
 
-// grid (groups of 64 heads, rows), sixteen warps.  The arithmetic and its order, hence the bits, are those of attn_tc_kernel (tiles of 128
-// keys, two partial score accumulators of 256 dims, sums over sixteen keys at a time), laid out for 64 heads:
+// grid (groups of 64 heads, rows), sixteen warps.  The arithmetic and its order, hence the bits, are those of attn_tc_kernel<32> (tiles of 128
+// keys, two partial score accumulators of 256 dims, sums over sixteen keys at a time; attn_tc_kernel<16> sums over eight), laid out for 64 heads:
 //   keys     thread = (key of the tile, 128 dims): quarter h = tid / 128 decodes slabs 2h and 2h + 1, and waits only for the value MMAs that
 //            read these two (output tile h), so the next tile's codes are widened under the last value MMAs
 //   scores   S[head, key] = Q K^T with M = 64: a head is a TMEM lane (sixteen per warp quarter), so the scores of 32 keys
@@ -666,8 +666,8 @@ constexpr int THREADS64 = 512;
 //            exchange of eight partial maxima and sums per head
 //   values   O^T[dim, head], as in attn_tc_kernel: four issuing threads, one 128-dim tile each
 // Shared memory holds one CTA per SM (K 128 KB, Q 64 KB, P 16 KB), so the phases of a tile follow each other; sixteen warps instead of eight
-// halve each thread's chain of loads, conversions and exponentials.  4,096 rows, 64 heads: a layer of
-// 128 window entries 615 -> 545 us, with 512 compressed ones 1,695 -> 1,267 us (553 and 1,358 with sixteen lanes of a warp in the softmax).
+// halve each thread's chain of loads, conversions and exponentials.  4,096 rows, 64 heads: a layer of 128 window entries 533 us, with 512 compressed
+// ones 1,275.  Of a window row's 17.7 us 6.5 pass until the first tile stands, 4.4 in scores, softmax and values, 6.9 in the epilogue; a further tile takes 6.7.
 __global__ void __launch_bounds__(THREADS64, 1) attn_tc64_kernel(AttnTcArgs a) {
   extern __shared__ uint8_t smem_raw[];
   AttnTc64Smem& S = *reinterpret_cast<AttnTc64Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);

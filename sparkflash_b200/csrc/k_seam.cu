@@ -369,8 +369,8 @@ __device__ unsigned long long g_fold_marks[4096 * 8];
 #endif
 
 // Four blocks per SM: what passes between the two loops is bf16 already and waits in the normalised row's place (shared memory, not registers), and that
-// place is the first partial's, which the same thread has read, unless the sum of the partials goes there.  Two blocks fitted before, by registers.
-// Bound by memory (105 KB a row): 4,096 rows of 5,120, four copies 150 -> 95 us, 777 rows 38 -> 25.
+// place is the first partial's, which the same thread has read, unless the sum of the partials goes there.  Bound by memory (105 KB a row): 4,096 rows of
+// 5,120, four copies 95 us, 777 rows 25; with two blocks per SM 150 and 38.
 template <int HC>
 __global__ void __launch_bounds__(FOLDR_THREADS, 4) seam_fold_rows_bulk_kernel(FoldArgs a) {
   extern __shared__ __align__(128) uint8_t fold_sm[];

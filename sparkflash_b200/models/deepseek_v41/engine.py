@@ -662,12 +662,13 @@ class Engine:
         return min(P, E_local + P // seg) + (n + seg - 1) // seg
 
     # From this many rows on, segments hold up to 64 pairs: an expert's weights then serve four times the rows, and the persistent kernels run.
-    # Steps of four layers over 64 / 128 experts, 16 pairs against 64: 64 rows 2.78 / 3.20 ms against 2.86 / 3.10, 100 rows 2.64 / 3.16 against
-    # 2.52 / 2.99, 200 rows 2.83 / 3.34 against 2.37 / 3.00, 500 rows 4.60 / 5.10 against 3.24 / 3.99.
+    # Captured steps of four layers over 64 / 128 experts and of two over 384, 16 pairs against 64: 48 rows 2.12 / 2.43 / 1.46 ms against 2.20 / 2.40 / 1.39,
+    # 100 rows 2.30 / 2.78 / 1.88 against 2.22 / 2.68 / 1.74, 200 rows 2.41 / 2.93 / 2.11 against 1.96 / 2.54 / 1.90, 511 rows 4.09 / 4.56 / 3.20
+    # against 2.67 / 3.36 / 2.76.
     GROUP_WIDE_ROWS = 100
-    # From this many pairs per expert on, 96: at 384 pairs gate/up takes 768 us instead of 836 and down 449 instead of 472; at 73 pairs, where one
-    # segment of 96 replaces two of 64, both read the weights from HBM at the same pace (222 / 225 and 130 / 128 us), and between 96 and 128 both
-    # sizes need two segments, the wider ones with a third more operand reads.
+    # From this many pairs per expert on, 96.  The same steps, 64 pairs against 96: over 64 experts 128 / 160 / 192 / 256 / 384 pairs per expert 5.34 / 6.47 /
+    # 7.62 / 10.20 / 14.98 ms against 5.25 / 6.49 / 7.41 / 9.78 / 14.69, over 128 experts 128 / 160 / 192 pairs 10.72 / 13.19 / 15.54 against 10.63 / 12.89 /
+    # 15.04.  Between 48 and 110 pairs they differ by -1 to 2 %, and at 24 pairs, where the wider tiles are three quarters empty, 96 takes 4 to 9 % longer.
     GROUP_WIDER_PAIRS = 128
 
     def _group_size(self, n: int, k: int, E: int) -> int:

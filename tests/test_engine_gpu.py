@@ -751,7 +751,8 @@ def test_wide_moe_segments_and_the_persistent_kernels_give_the_bits_of_16_pair_s
 
 @pytest.mark.parametrize("rows", [5, 96, 97, 128])
 def test_moe_segments_of_96_pairs_give_the_bits_of_16_pair_segments(tiny, rows):
-    """The shared expert's rows fill one segment, or end a row before or after its border; the routed experts' segments are never full."""
+    """The shared expert's rows fill one segment, or end a row before or after its border; the routed experts' segments are never full (experts with
+    several full ones: test_bulk_kernels_gpu.py)."""
     from sparkflash_b200.models.deepseek_v41 import engine as E
     cfg, ck, w, orc, dw = tiny
     prompt, outs = _prompt(cfg, rows, seed=29), []
