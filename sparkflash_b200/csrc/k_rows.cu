@@ -27,31 +27,6 @@ namespace sfb {
 namespace rows {
 
 // ---- seam ------------------------------------------------------------------------------------------------------------
-struct SeamArgs {
-  float* x;                 // [rows, d] residual, 32-bit
-  const void* y;            // [rows, d] sublayer output (T) or null: no residual update
-  const void* y2;           // second branch (T) or null
-  const float *mw, *mw2;    // RMS weights of the two branches
-  const float* parts_w;     // [rows, parts]: y is [rows, parts, d] and the output their weighted sum; or null
-  const float *pw, *pb;     // post-norm (pb null: no bias), or the scale
-  const void* embed;        // [vocab, d] (T)
-  const int* tokens;        // [rows]
-  const float* step_vec;    // [d] or null: added after the update
-  float* tap;               // [rows, d] or null: the residual right after the update
-  const float *nw, *nb;     // next norm, or null: h is the residual itself
-  void* h;                  // [rows, d] (T) its output, or null
-  const int* row_map;       // null: row = block; otherwise the residual row of output row `block`
-  const float* cw;          // [taps, d] input convolution, or null
-  void* hist;               // [slots, taps - 1, d] (T)
-  const int *src, *dst;     // [rows] state versions of single-row segments
-  int from_embed, add_embed, taps, d, vocab;
-  int parts, post, rms;     // post: POST_*; rms: the next norm is an RMS norm
-  float eps, embed_scale;
-  Status* status;
-};
-
-constexpr int POST_LAYER = 0, POST_RMS = 1, POST_SCALE = 2;
-
 // Mean and sum of squared deviations of a row held as x[NV][V] per thread (`wcnt` = how many of the elements are this warp's):
 // each warp takes both about its own mean, then the warps' pairs are combined - one barrier.
 template <int V, int NV>
@@ -931,6 +906,8 @@ int sfb_rows_seam(void* x, const void* y, const void* y2, const void* mw, const 
              (float*)tap, (const float*)nw, (const float*)nb, h, row_map, (const float*)cw, hist, src, dst, from_embed, add_embed, taps, d,
              vocab, parts, post, rms, eps, embed_scale, (Status*)status};
   if (fp32) return d % 4 ? launch_seam<float, 1>(a, n, stream) : launch_seam<float, 4>(a, n, stream);
+  const int rc = seam_many(a, n, stream);
+  if (rc >= 0) return rc;
   return d % 4 ? launch_seam<__nv_bfloat16, 1>(a, n, stream) : launch_seam<__nv_bfloat16, 4>(a, n, stream);
 }
 

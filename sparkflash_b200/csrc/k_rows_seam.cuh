@@ -1,9 +1,42 @@
-// What the seam kernels of the layered decoders share (k_rows.cu: one residual; k_rows_streams.cu: several streams of it).
+// What the seam kernels of the layered decoders share (k_rows.cu, many rows k_rows_seam_many.cu: one residual; k_rows_streams.cu: several streams of it).
 #pragma once
 #include "k_rows.cuh"
 
 namespace sfb {
 namespace rows {
+
+// one residual (k_rows.cu, k_rows_seam_many.cu)
+struct SeamArgs {
+  float* x;                 // [rows, d] residual, 32-bit
+  const void* y;            // [rows, d] sublayer output (T) or null: no residual update
+  const void* y2;           // second branch (T) or null
+  const float *mw, *mw2;    // RMS weights of the two branches
+  const float* parts_w;     // [rows, parts]: y is [rows, parts, d] and the output their weighted sum; or null
+  const float *pw, *pb;     // post-norm (pb null: no bias), or the scale
+  const void* embed;        // [vocab, d] (T)
+  const int* tokens;        // [rows]
+  const float* step_vec;    // [d] or null: added after the update
+  float* tap;               // [rows, d] or null: the residual right after the update
+  const float *nw, *nb;     // next norm, or null: h is the residual itself
+  void* h;                  // [rows, d] (T) its output, or null
+  const int* row_map;       // null: row = block; otherwise the residual row of output row `block`
+  const float* cw;          // [taps, d] input convolution, or null
+  void* hist;               // [slots, taps - 1, d] (T)
+  const int *src, *dst;     // [rows] state versions of single-row segments
+  int from_embed, add_embed, taps, d, vocab;
+  int parts, post, rms;     // post: POST_*; rms: the next norm is an RMS norm
+  float eps, embed_scale;
+  Status* status;
+};
+
+constexpr int POST_LAYER = 0, POST_RMS = 1, POST_SCALE = 2;
+
+// From two rows per SM on, of 2,048 elements (from 2,048 rows on 1,024) and more, the seam is the persistent kernel of k_rows_seam_many.cu.  0 or an error; -1: it
+// does not take these.
+constexpr int SEAM_MANY_ROWS = 297;
+int seam_many(const SeamArgs& a, int n, cudaStream_t stream);
+
+
 
 // Input convolution of a step of single-row segments: o (channels c .. of a norm's output) becomes o + conv(o) over the carried inputs hs
 // (null: zeros), whose next version is hd.  `ahead`: weights and carried inputs are held in registers (rw, rg: [taps][i][V]).

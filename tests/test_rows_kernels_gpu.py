@@ -70,6 +70,38 @@ def test_seam_norms_merge_embedding_and_step_vector(dt, d):
     assert st.tolist()[0] == 2 and st.tolist()[2] == V          # a token outside the table is reported, not read
 
 
+@pytest.mark.parametrize("form", ["layer", "rms", "scale", "plain", "merged", "parts1", "parts9", "norm"])
+@pytest.mark.parametrize("n,d", [(296, 2048), (297, 2048), (445, 2056), (1037, 3000), (299, 4096), (297, 4104), (2048, 1024), (2047, 1024), (2050, 1032), (400, 264)])
+def test_seam_of_many_rows(n, d, form):
+    """Around the sizes of the persistent kernel: fewest rows and one less, widths that fill a group of warps and that do not, the widest and the
+    next one beyond, the narrowest; against 64 bits.  x: 32-bit sums of terms up to 8; h: the rounding to bf16."""
+    g = torch.Generator().manual_seed(n + d)
+    r = lambda *s: torch.randn(*s, generator=g)
+    eps, dt = 1e-4, torch.bfloat16
+    x, y, y2, z, wt = r(n, d), r(n, d).to(dt) + 1, r(n, d).to(dt), r(n, int(form[5:] or 1) if form[:5] == "parts" else 1, d).to(dt), torch.rand(n, 9, generator=g)[:, :int(form[5:]) if form[:5] == "parts" else 1]
+    w, b = [1 + 0.3 * r(d) for _ in range(4)], [0.3 * r(d) for _ in range(2)]
+    c = lambda t: t.to("cuda").contiguous()
+    ln = lambda t, a, o: torch.nn.functional.layer_norm(t, (d,), a.double(), None if o is None else o.double(), eps)
+    rms = lambda t, a: t * torch.rsqrt((t * t).mean(-1, keepdim=True) + eps) * a.double()
+    X, Y = x.double(), y.double()
+    want_x, kw = {"layer": lambda: (X + ln(Y, w[0], b[0]), dict(y=c(y), post=(c(w[0]), c(b[0])), norm=(c(w[1]), c(b[1])))),
+                  "rms": lambda: (X + rms(Y, w[0]), dict(y=c(y), post=(c(w[0]), None), post_kind="rms", norm=(c(w[1]), None), norm_kind="rms")),
+                  "scale": lambda: (X + Y * w[0].double(), dict(y=c(y), post=(c(w[0]), None), post_kind="scale", norm=(c(w[1]), None), norm_kind="rms")),
+                  "plain": lambda: (X + ln(Y, w[0], None), dict(y=c(y), post=(c(w[0]), None))),
+                  "merged": lambda: (X + ln(0.5 * (rms(Y, w[2]) + rms(y2.double(), w[3])), w[0], b[0]),
+                                     dict(y=c(y), y2=c(y2), merge_w=(c(w[2]), c(w[3])), post=(c(w[0]), c(b[0])), norm=(c(w[1]), c(b[1])))),
+                  "norm": lambda: (X, dict(norm=(c(w[1]), c(b[1]))))}.get(
+        form, lambda: (X + (z.double() * wt.double()[..., None]).sum(1) * w[0].double(),
+                       dict(y=c(z), parts_w=c(wt), post=(c(w[0]), None), post_kind="scale", norm=(c(w[1]), None), norm_kind="rms")))()
+    norm = kw.get("norm")
+    want_h = want_x if norm is None else rms(want_x, w[1]) if kw.get("norm_kind") == "rms" else ln(want_x, w[1], b[1])
+    xs, h, st = c(x), torch.zeros(n, d, dtype=dt, device="cuda"), _status()
+    R.seam(xs, n, h=h, eps=eps, status=st, **kw)
+    assert st.tolist()[0] == 0
+    assert (xs.cpu().double() - want_x).abs().max() < 4e-5
+    assert ((h.cpu().double() - want_h).abs() < 2 ** -8 * want_h.abs() + 4e-5).all()
+
+
 @pytest.mark.parametrize("dt", DTYPES)
 @pytest.mark.parametrize("taps,C", [(1, 24), (2, 40), (3, 33), (4, 512), (7, 20)])
 def test_conv_portions_carry_their_inputs(dt, taps, C):
