@@ -43,6 +43,13 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostArgs a) {
   const int row = blockIdx.x;
   const __nv_bfloat16* raw = a.raw + (size_t)row * (a.q + a.hd);
   float ss = 0.f, rs;
+  // the norm's weights, which nothing before this kernel writes, are here by the time the sum is: up to 2,048 of them
+  constexpr int AHEAD = 8;
+  const float* nw = blockIdx.y == 0 ? a.q_norm_w : a.kv_norm_w;
+  const int width = blockIdx.y == 0 ? a.q : a.hd;
+  float w[AHEAD];
+#pragma unroll
+  for (int k = 0; k < AHEAD; ++k) w[k] = threadIdx.x + k * 256 < width ? nw[threadIdx.x + k * 256] : 0.f;
   pdl_launch_dependents();
   pdl_wait();
   if (blockIdx.y == 0) {
@@ -50,9 +57,8 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostArgs a) {
   for (int i = threadIdx.x; i < a.q; i += 256) { float v = bf16_to_f(raw[i]); buf[i] = v; ss += v * v; }
   ss = block_sum(ss, sh);
   rs = rsqrtf(ss / (float)a.q + a.eps);
-  for (int i0 = (threadIdx.x >> 5) * 32; i0 < a.q; i0 += 256) {
-    const int i = i0 + (threadIdx.x & 31);
-    float v = bfr(buf[i] * rs * a.q_norm_w[i]);
+  auto put = [&](int i, float weight) {      // q is a multiple of 32: whole warps
+    float v = bfr(buf[i] * rs * weight);
     if (a.qr_b) a.qr_b[(size_t)row * a.q + i] = __float2bfloat16_rn(v);
     uint8_t sc;
     uint8_t qv = warp_quant_fp8(v, &sc);
@@ -61,7 +67,11 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostArgs a) {
       a.qr_s[(size_t)row * (a.q / 32) + i / 32] = sc;
       if (a.qr_atom) a.qr_atom[sf_offset(row, i / 32, a.q / 32)] = sc;
     }
-  }
+  };
+#pragma unroll
+  for (int k = 0; k < AHEAD; ++k)
+    if (threadIdx.x + k * 256 < a.q) put(threadIdx.x + k * 256, w[k]);
+  for (int i = threadIdx.x + AHEAD * 256; i < a.q; i += 256) put(i, nw[i]);
   return;
   }
   // ---- kv_norm + rope + fp8 + window append ----
@@ -70,7 +80,10 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostArgs a) {
   for (int i = threadIdx.x; i < a.hd; i += 256) { float v = bf16_to_f(raw[a.q + i]); buf[i] = v; ss += v * v; }
   ss = block_sum(ss, sh);
   rs = rsqrtf(ss / (float)a.hd + a.eps);
-  for (int i = threadIdx.x; i < a.hd; i += 256) buf[i] = bfr(buf[i] * rs * a.kv_norm_w[i]);
+#pragma unroll
+  for (int k = 0; k < AHEAD; ++k)
+    if (threadIdx.x + k * 256 < a.hd) buf[threadIdx.x + k * 256] = bfr(buf[threadIdx.x + k * 256] * rs * w[k]);
+  for (int i = threadIdx.x + AHEAD * 256; i < a.hd; i += 256) buf[i] = bfr(buf[i] * rs * nw[i]);
   __syncthreads();
   const int r0 = a.hd - a.rd;
   for (int p = threadIdx.x; p < a.rd / 2; p += 256) {

@@ -30,30 +30,41 @@ struct RouterArgs {
   float route_scale;
 };
 
+// One block per row.  All four warps make the scores; the choice, a chain of k maxima, is one warp's, without a barrier in it.
 __global__ void __launch_bounds__(128) router_topk_kernel(RouterArgs a) {
   extern __shared__ float sm[];
   float* s = sm;            // [E] scores
   float* key = sm + a.E;    // [E] selection keys
-  __shared__ float rv[4];
-  __shared__ int ri[4];
-  __shared__ int pick[16];
-  const int row = blockIdx.x;
+  __shared__ float chosen[16];
+  const int row = blockIdx.x, lane = threadIdx.x & 31;
+  const bool image = a.is_image && a.bias_vl;
+  constexpr int AHEAD = 4;
+  float b[AHEAD];           // the text bias, which nothing before this kernel writes
+#pragma unroll
+  for (int i = 0; i < AHEAD; ++i) b[i] = threadIdx.x + i * 128 < a.E ? a.bias[threadIdx.x + i * 128] : 0.f;
   pdl_launch_dependents();
   pdl_wait();
-  const float* bias = (a.is_image && a.bias_vl && a.is_image[row]) ? a.bias_vl : a.bias;
-  for (int e = threadIdx.x; e < a.E; e += 128) {
+  const float* other = image && a.is_image[row] ? a.bias_vl : nullptr;
+  auto score = [&](int e, float bias) {
     float x = 0.f;
     for (int z = 0; z < a.nsplit; ++z) x += a.dots[(size_t)z * a.split_stride + (size_t)row * a.E + e];
     float sp = x > 20.f ? x : log1pf(expf(x));
     float v = sqrtf(sp);
     s[e] = v;
-    key[e] = v + bias[e];
-  }
+    key[e] = v + (other ? other[e] : bias);
+  };
+#pragma unroll
+  for (int i = 0; i < AHEAD; ++i)
+    if (threadIdx.x + i * 128 < a.E) score(threadIdx.x + i * 128, b[i]);
+  for (int e = threadIdx.x + AHEAD * 128; e < a.E; e += 128) score(e, a.bias[e]);
   __syncthreads();
+  if (threadIdx.x >= 32) return;
+  int mine = 0;             // lane t: the t-th choice
   for (int t = 0; t < a.k; ++t) {
     float bv = -INFINITY;
     int bi = 0x7fffffff;
-    for (int e = threadIdx.x; e < a.E; e += 128) {
+#pragma unroll 4
+    for (int e = lane; e < a.E; e += 32) {
       float v = key[e];
       if (v > bv || (v == bv && e < bi)) { bv = v; bi = e; }
     }
@@ -63,28 +74,23 @@ __global__ void __launch_bounds__(128) router_topk_kernel(RouterArgs a) {
       int oi = __shfl_xor_sync(0xffffffffu, bi, o);
       if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
     }
-    if ((threadIdx.x & 31) == 0) { rv[threadIdx.x >> 5] = bv; ri[threadIdx.x >> 5] = bi; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int w = 1; w < 4; ++w)
-        if (rv[w] > bv || (rv[w] == bv && ri[w] < bi)) { bv = rv[w]; bi = ri[w]; }
-      pick[t] = bi;
-      key[bi] = -INFINITY;
-    }
-    __syncthreads();
+    bi = min(bi, a.E - 1);  // no score is a number
+    if (lane == t) mine = bi;
+    if (lane == (bi & 31)) key[bi] = -INFINITY;
+    __syncwarp();
   }
-  if (threadIdx.x == 0) {
-    for (int i = 1; i < a.k; ++i) {  // ascending ids
-      int v = pick[i], j = i - 1;
-      while (j >= 0 && pick[j] > v) { pick[j + 1] = pick[j]; --j; }
-      pick[j + 1] = v;
-    }
-    float sum = 0.f;
-    for (int i = 0; i < a.k; ++i) sum += s[pick[i]];
-    for (int i = 0; i < a.k; ++i) {
-      a.ids[(size_t)row * a.k + i] = pick[i];
-      a.wts[(size_t)row * a.k + i] = s[pick[i]] / (sum + 1e-20f) * a.route_scale;
-    }
+  int place = 0;            // ascending ids
+  for (int j = 0; j < a.k; ++j) {
+    const int other_id = __shfl_sync(0xffffffffu, mine, j);
+    place += other_id < mine || (other_id == mine && j < lane);
+  }
+  if (lane < a.k) chosen[place] = s[mine];
+  __syncwarp();
+  float sum = 0.f;
+  for (int i = 0; i < a.k; ++i) sum += chosen[i];
+  if (lane < a.k) {
+    a.ids[(size_t)row * a.k + place] = mine;
+    a.wts[(size_t)row * a.k + place] = s[mine] / (sum + 1e-20f) * a.route_scale;
   }
 }
 

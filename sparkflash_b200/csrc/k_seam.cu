@@ -78,6 +78,13 @@ __global__ void __cluster_dims__(FOLD_CLUSTER, 1, 1) __launch_bounds__(FOLD_THRE
   const int c_lo = rank * cpc;
   __shared__ float part_ss, part_hss;
   __shared__ float sh[32];
+  // weights of the norm: nothing before this kernel writes them
+  float nw[FOLD_MAX_IT];
+#pragma unroll
+  for (int it = 0; it < FOLD_MAX_IT; ++it) {
+    const int lc = it * FOLD_THREADS + threadIdx.x;
+    nw[it] = lc < cpc ? a.norm_w[c_lo + lc] : 0.f;
+  }
   pdl_launch_dependents();
   pdl_wait();
   float hsq = 0.f;
@@ -164,7 +171,7 @@ __global__ void __cluster_dims__(FOLD_CLUSTER, 1, 1) __launch_bounds__(FOLD_THRE
     // whole warps are in or out of range (cpc and FOLD_THREADS are multiples of 32)
     if (lc - lane < cpc) {
       const int col = c_lo + lc;
-      const float v = bfr(xh[it] * rsx * a.norm_w[col]);
+      const float v = bfr(xh[it] * rsx * nw[it]);
       if (a.xn) a.xn[(size_t)row * d + col] = __float2bfloat16_rn(v);
       if (a.xq) {
         uint8_t sc;

@@ -823,3 +823,53 @@ def test_guard_bands_stay_intact_over_a_many_row_step_at_full_per_token_shapes()
         tok = eng.step(ids[1200:1201], [0], [1200])
     eng.check_status()
     assert 0 <= int(tok[0]) < cfg.vocab_size and len(eng.guard_arena.records) > 40
+
+
+@pytest.mark.parametrize("E,k", [(6, 6), (24, 1), (33, 4), (64, 6), (384, 6), (512, 16), (520, 8), (1000, 16)])
+def test_router_choice_at_its_edges(E, k):
+    """Fewer experts than lanes, experts beyond the biases held ahead, every expert chosen, the most choices; equal scores go to the lower id; rows of images take
+    the other bias."""
+    from sparkflash_b200.ops import native as N
+    g = torch.Generator().manual_seed(E)
+    n = 5
+    dots, bias, other = (torch.randn(n, E, generator=g) * 2).round(decimals=1), (torch.randn(E, generator=g) * 0.1).round(decimals=1), torch.randn(E, generator=g)
+    dots[1] = 0.5
+    bias[:E // 2] = 0
+    image = torch.tensor([0, 0, 1, 0, 1], dtype=torch.uint8)
+    ids, wts = torch.full((n, k), -9, dtype=torch.int32, device="cuda"), torch.zeros(n, k, device="cuda")
+    N.router_topk(dots.cuda(), bias.cuda(), other.cuda(), image.cuda(), ids, wts, n, E, k, 1.5)
+    s = torch.sqrt(torch.nn.functional.softplus(dots.double()))
+    for r in range(n):
+        key = s[r] + (other if image[r] else bias).double()
+        got = ids[r].tolist()
+        assert got == sorted(set(got)) and 0 <= got[0] and got[-1] < E
+        rest = [e for e in range(E) if e not in got]
+        if rest:
+            assert key[got].min() >= key[rest].max() - 1e-5
+            assert all(not (e < c and abs(float(key[e] - key[c])) == 0) for c in got for e in rest)      # equal keys: the lower id
+        w = s[r][got] / (s[r][got].sum() + 1e-20) * 1.5
+        assert torch.allclose(wts[r].cpu().double(), w, rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("q,hd,rd", [(64, 64, 32), (1280, 512, 64), (2048, 128, 64), (2080, 2112, 64)])
+def test_query_and_key_norms_with_weights_held_ahead(q, hd, rd):
+    """Widths below, at and beyond the 2,048 weights that are fetched before the previous kernel's end."""
+    from sparkflash_b200.ops import native as N
+    g = torch.Generator().manual_seed(q)
+    n, ring, dev, eps = 3, 16, "cuda", 1e-6
+    raw = (torch.randn(n, q + hd, generator=g) * 2).to(torch.bfloat16)
+    qw, kw = 1 + 0.3 * torch.randn(q, generator=g), 1 + 0.3 * torch.randn(hd, generator=g)
+    rope = torch.zeros(n, rd // 2, 2, device=dev)
+    rope[..., 0] = 1
+    lane, pos = torch.tensor([0, 1, 0], dtype=torch.int32, device=dev), torch.tensor([3, 20, 4], dtype=torch.int32, device=dev)
+    qq, qs = torch.zeros(n, q, dtype=torch.uint8, device=dev), torch.zeros(n, q // 32, dtype=torch.uint8, device=dev)
+    wq, ws = torch.zeros(2, ring, hd, dtype=torch.uint8, device=dev), torch.zeros(2, ring, hd // 32, dtype=torch.uint8, device=dev)
+    N.qkv_post(raw.to(dev), qw.to(dev), kw.to(dev), rope, lane, pos, qq, qs, wq, ws, n, q, hd, rd, ring, eps)
+    norm = lambda x, w: (x * torch.rsqrt((x * x).mean(-1, keepdim=True) + eps) * w)
+    x = raw.double()
+    want_q, want_k = norm(x[:, :q], qw.double()), norm(x[:, q:], kw.double())
+    got_q = C.act_dequant_fp8(qq.cpu(), qs.cpu()).double()
+    got_k = torch.stack([C.act_dequant_fp8(wq[l, p % ring][None].cpu(), ws[l, p % ring][None].cpu())[0] for l, p in zip(lane.tolist(), pos.tolist())]).double()
+    for got, want in ((got_q, want_q), (got_k, want_k)):      # E4M3: 2^-4 of a value, 2^-9 of its group's largest scale step
+        top = want.abs().unflatten(-1, (-1, 32)).amax(-1, keepdim=True).expand(-1, -1, 32).flatten(1)
+        assert ((got - want).abs() <= 2 ** -4 * want.abs() * 1.1 + 2 ** -9 * top).all()
