@@ -36,6 +36,29 @@ constexpr int POST_LAYER = 0, POST_RMS = 1, POST_SCALE = 2;
 constexpr int SEAM_MANY_ROWS = 297;
 int seam_many(const SeamArgs& a, int n, cudaStream_t stream);
 
+// several streams of the residual (k_rows_streams.cu, k_rows_seam_many.cu)
+struct StreamArgs {
+  float* x;                 // [rows, S, d] streams
+  const void* y;            // [rows, d] sublayer output (T) or null: no update
+  const float* parts_w;     // [rows, parts]: y is [rows, parts, d] and the output their weighted sum; or null
+  const float *mix, *out;   // [S, S] from, to; [S]
+  const void* embed;        // [vocab, d] (T): the row begins with it (y null)
+  const int* tokens;        // [rows]
+  float* tap;               // [rows, d] or null: the sum of the new streams
+  const float* in;          // [S] or null: ones
+  const float* nw;          // [d]
+  void* h;                  // [rows, d] (T)
+  const int* row_map;       // null: row = block; otherwise the residual row of output row `block`
+  const float* cw;          // [taps, d] input convolution, or null
+  void* hist;               // [slots, taps - 1, d] (T)
+  const int *src, *dst;     // [rows] state versions of single-row segments
+  int S, d, parts, taps, vocab, keep;    // keep: the streams are stored
+  float eps, embed_scale;
+  Status* status;
+};
+// two to four streams of 1,024 and more elements, as seam_many
+int streams_many(const StreamArgs& a, int n, cudaStream_t stream);
+
 
 
 // Input convolution of a step of single-row segments: o (channels c .. of a norm's output) becomes o + conv(o) over the carried inputs hs

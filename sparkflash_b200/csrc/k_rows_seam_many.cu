@@ -277,6 +277,202 @@ __global__ void __launch_bounds__(64 + 768, 1) seam_many_kernel(SeamMany m) {
   if (tid == 0 && *dead) status_set(a.status, ST_TIMEOUT, 78, blockIdx.x, 0);
 }
 
+// The same for S streams: k_rows_streams.cu's sums, a row of all streams a stage.  Four streams, us (floor): 3,000 x 2,048 47 -> 35 (34), with four parts 73 -> 41 (39); 600 x 2,048
+// 16 -> 14 and 23 -> 16; 3,000 x 3,000 67 -> 52 (49) and 149 -> 66 (58); 3,000 x 1,024 23 -> 21 and 35 -> 23; 300 x 1,024 9 -> 10 and 11 -> 10.  Four streams of 4,096
+// do not fit three stages and keep the block per row.
+struct StreamsMany {
+  StreamArgs a;
+  int n, stages, groups, threads;
+  uint32_t load, stage, weights;
+};
+
+template <int S, int NV>
+__global__ void __launch_bounds__(64 + 512, 1) streams_many_kernel(StreamsMany m) {
+  using T = __nv_bfloat16;
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ ManyBars B;
+  const StreamArgs& a = m.a;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, d = a.d, parts = a.parts_w ? a.parts : 1;
+  volatile int* dead = &B.dead;
+  uint8_t* ring = smem + m.weights;
+  if (tid == 0) {
+    B.dead = 0;
+    for (int i = 0; i < m.stages; ++i) { tc::mbar_init(&B.full[i], 1); tc::mbar_init(&B.done[i], m.threads / 32); tc::mbar_init(&B.empty[i], 1); }
+    tc::mbar_init(&B.weights, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  for (int i = tid; i < MANY_MAX_GROUPS * 48; i += blockDim.x) (&B.sums[0][0][0])[i] = 0.f;
+  pdl_launch_dependents();
+  __syncthreads();
+  if (warp == 0) {
+    if (elect_one()) {
+      tc::mbar_expect(&B.weights, m.weights);
+      bulk_in(smem, a.nw, d * 4, &B.weights);
+      pdl_wait();
+      int k = 0;
+      for (int r = blockIdx.x; r < m.n; r += gridDim.x, ++k) {
+        const int st = k % m.stages;
+        if (k >= m.stages && !tc::mbar_wait(&B.empty[st], (k / m.stages - 1) & 1, dead)) break;
+        tc::mbar_expect(&B.full[st], m.load);
+        uint8_t* p = ring + (size_t)st * m.stage;
+        bulk_in(p, a.x + (size_t)r * S * d, S * d * 4, &B.full[st]);
+        bulk_in(p + S * d * 4, (const T*)a.y + (size_t)r * parts * d, parts * d * 2, &B.full[st]);
+      }
+      if (*dead)                 // copies still in flight must land before the CTA ends
+        for (int j = max(0, k - m.stages); j < k; ++j)
+          for (int i = 0; i < 100000 && !tc::mbar_try(&B.full[j % m.stages], (j / m.stages) & 1); ++i) __nanosleep(64);
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      pdl_wait();
+      int k = 0;
+      for (int r = blockIdx.x; r < m.n; r += gridDim.x, ++k) {
+        const int st = k % m.stages;
+        if (!tc::mbar_wait(&B.done[st], (k / m.stages) & 1, dead)) break;
+        const uint8_t* p = ring + (size_t)st * m.stage;
+        if (a.keep) bulk_out(a.x + (size_t)r * S * d, p, S * d * 4);
+        bulk_out((T*)a.h + (size_t)r * d, p + S * d * 4, d * 2);
+        tc::bulk_commit();
+        asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        if (k > 0) tc::mbar_arrive(&B.empty[(k - 1) % m.stages]);
+      }
+      tc::bulk_wait_read();
+    }
+  } else {
+    const int g = (tid - 64) / m.threads, t0 = (tid - 64) % m.threads, w = t0 >> 5;
+    const int step = m.threads * 4, c0 = t0 * 4;
+    float mix[S][S], out[S], in[S];
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      in[s] = a.in ? a.in[s] : 1.f;
+      out[s] = a.out[s];
+#pragma unroll
+      for (int t = 0; t < S; ++t) mix[s][t] = a.mix[s * S + t];
+    }
+    const float* nw = reinterpret_cast<const float*>(smem);
+    bool ok = tc::mbar_wait(&B.weights, 0, dead);
+    pdl_wait();
+    int k = g, phase = 0;
+    for (int r = blockIdx.x + g * gridDim.x; ok && r < m.n; r += m.groups * gridDim.x, k += m.groups) {
+      const int st = k % m.stages;
+      float wj[8];
+      if (a.parts_w) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) wj[j] = j < a.parts ? a.parts_w[(size_t)r * a.parts + j] : 0.f;
+      }
+      if (lane == 0) ok = tc::mbar_wait(&B.full[st], (k / m.stages) & 1, dead);
+      ok = __shfl_sync(0xffffffffu, ok, 0);
+      if (!ok) break;
+      float* xs = reinterpret_cast<float*>(ring + (size_t)st * m.stage);
+      T* ys = reinterpret_cast<T*>(xs + S * d);
+      float u[NV][4], ss = 0.f;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int c = c0 + i * step;
+        if (c >= d) continue;
+        float y[4], x[S][4];
+        if (a.parts_w) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) y[q] = 0.f;
+          for (int j = 0; j < a.parts; ++j) {
+            float f = j < 8 ? 0.f : a.parts_w[(size_t)r * a.parts + j], z[4];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) if (j == q) f = wj[q];
+            load_v<T, 4>(ys + (size_t)j * d + c, z);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) y[q] = fmaf(f, z[q], y[q]);
+          }
+        } else {
+          load_v<T, 4>(ys + c, y);
+        }
+#pragma unroll
+        for (int s = 0; s < S; ++s) load_v<float, 4>(xs + s * d + c, x[s]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) u[i][q] = 0.f;
+#pragma unroll
+        for (int t = 0; t < S; ++t) {
+          float n[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            n[q] = out[t] * y[q];
+#pragma unroll
+            for (int s = 0; s < S; ++s) n[q] = fmaf(mix[s][t], x[s][q], n[q]);
+            u[i][q] = fmaf(in[t], n[q], u[i][q]);
+          }
+          if (a.keep) store_v<float, 4>(xs + t * d + c, n);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < NV; ++i)
+        if (c0 + i * step < d) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) ss = fmaf(u[i][q], u[i][q], ss);
+        }
+      float* s = B.sums[g][phase++ & 1];
+      ss = warp_sum(ss);
+      if (lane == 0) s[w] = ss;
+      group_sync(g, m.threads);
+      ss = sum8(s);
+      const float rs = 1.f / sqrtf(ss / (float)d + a.eps);
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int c = c0 + i * step;
+        if (c >= d) continue;
+        float o[4], f[4];
+        load_v<float, 4>(nw + c, f);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) o[q] = u[i][q] * rs * f[q];
+        store_v<T, 4>(ys + c, o);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&B.done[st]);
+    }
+  }
+  __syncthreads();
+  if (tid == 0 && *dead) status_set(a.status, ST_TIMEOUT, 80, blockIdx.x, 0);
+}
+
+static int sm_count() {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+template <int S, int NV>
+static int launch_streams_many(const StreamsMany& m, cudaStream_t stream) {
+  static bool done = false;
+  if (!done) {
+    const cudaError_t e = cudaFuncSetAttribute(streams_many_kernel<S, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, MANY_SMEM);
+    if (e != cudaSuccess) return (int)e;
+    done = true;
+  }
+  const int sms = sm_count();
+  return (int)sfb_launch(streams_many_kernel<S, NV>, dim3(m.n < sms ? m.n : sms), dim3(64 + m.groups * m.threads), m.weights + m.stages * m.stage, stream, m);
+}
+
+int streams_many(const StreamArgs& a, int n, cudaStream_t stream) {
+  const int d = a.d;
+  if (n < SEAM_MANY_ROWS || !a.y || a.tap || a.row_map || a.cw || a.S < 2 || a.S > 4 || d % 8 || d > 4096 || d < 1024) return -1;
+  if (((uintptr_t)a.x | (uintptr_t)a.y | (uintptr_t)a.nw | (uintptr_t)a.h) % 16) return -1;
+  StreamsMany m{};
+  m.a = a; m.n = n;
+  const int parts = a.parts_w ? a.parts : 1;
+  m.weights = d * 4;
+  m.load = a.S * d * 4 + parts * d * 2;
+  m.stage = (m.load + 127) & ~127u;
+  if ((long long)m.weights + 3ll * m.stage > MANY_SMEM) return -1;
+  m.stages = (int)((MANY_SMEM - m.weights) / m.stage);
+  if (m.stages > MANY_MAX_STAGES) m.stages = MANY_MAX_STAGES;
+  int nv = 1;              // as launch_streams spreads a row
+  while (nv < 4 && (d / 4 + nv - 1) / nv > (nv >= 2 ? 256 : 128)) nv *= 2;
+  m.threads = ((d / 4 + nv - 1) / nv + 31) / 32 * 32;
+  m.groups = 512 / m.threads;
+  if (m.groups > m.stages - 1) m.groups = m.stages - 1;
+  if (nv <= 2) return a.S == 2 ? launch_streams_many<2, 2>(m, stream) : a.S == 3 ? launch_streams_many<3, 2>(m, stream) : launch_streams_many<4, 2>(m, stream);
+  return a.S == 2 ? launch_streams_many<2, 4>(m, stream) : a.S == 3 ? launch_streams_many<3, 4>(m, stream) : launch_streams_many<4, 4>(m, stream);
+}
+
 // Not: fewer rows, the ends of a forward (embedding, chosen rows), convolutions of single rows, rows that are not whole 16-byte words or do not fit.
 int seam_many(const SeamArgs& a, int n, cudaStream_t stream) {
   const int d = a.d;
@@ -306,9 +502,7 @@ int seam_many(const SeamArgs& a, int n, cudaStream_t stream) {
     if (e != cudaSuccess) return (int)e;
     done = true;
   }
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   return (int)sfb_launch(seam_many_kernel<MANY_NV>, dim3(n < sms ? n : sms), dim3(64 + m.groups * m.threads), m.weights + m.stages * m.stage, stream, m);
 }
 

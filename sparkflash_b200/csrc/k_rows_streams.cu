@@ -12,26 +12,6 @@
 namespace sfb {
 namespace rows {
 
-struct StreamArgs {
-  float* x;                 // [rows, S, d] streams
-  const void* y;            // [rows, d] sublayer output (T) or null: no update
-  const float* parts_w;     // [rows, parts]: y is [rows, parts, d] and the output their weighted sum; or null
-  const float *mix, *out;   // [S, S] from, to; [S]
-  const void* embed;        // [vocab, d] (T): the row begins with it (y null)
-  const int* tokens;        // [rows]
-  float* tap;               // [rows, d] or null: the sum of the new streams
-  const float* in;          // [S] or null: ones
-  const float* nw;          // [d]
-  void* h;                  // [rows, d] (T)
-  const int* row_map;       // null: row = block; otherwise the residual row of output row `block`
-  const float* cw;          // [taps, d] input convolution, or null
-  void* hist;               // [slots, taps - 1, d] (T)
-  const int *src, *dst;     // [rows] state versions of single-row segments
-  int S, d, parts, taps, vocab, keep;    // keep: the streams are stored
-  float eps, embed_scale;
-  Status* status;
-};
-
 // SM: most streams.  AHEAD (few rows): weights and the convolution's carried inputs are requested before they are needed.
 template <typename T, int V, int NV, int SM, bool AHEAD>
 __global__ void __launch_bounds__(NV < 4 ? 256 : 512) stream_seam_kernel(StreamArgs a) {
@@ -230,6 +210,8 @@ int sfb_rows_streams(void* x, const void* y, const void* parts_w, const void* mi
   StreamArgs a{(float*)x, y, (const float*)parts_w, (const float*)mix, (const float*)out, embed, tokens, (float*)tap, (const float*)in, (const float*)nw, h, row_map,
                (const float*)cw, hist, src, dst, streams, d, parts, taps, vocab, keep, eps, embed_scale, (Status*)status};
   if (fp32) return d % 4 ? launch_streams<float, 1>(a, n, stream) : launch_streams<float, 4>(a, n, stream);
+  const int rc = streams_many(a, n, stream);
+  if (rc >= 0) return rc;
   return d % 4 ? launch_streams<__nv_bfloat16, 1>(a, n, stream) : launch_streams<__nv_bfloat16, 4>(a, n, stream);
 }
 

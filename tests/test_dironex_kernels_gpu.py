@@ -376,3 +376,23 @@ def test_one_key_stands_out_anywhere_in_a_long_context(H, rank, rot, dt):
             off = (c.float().view(-1, H, rank) - want).abs().amax((1, 2))
             for p, o in zip(rows, off.tolist()):
                 assert (o < 0.05) == (p >= at), (at, p, o)
+
+
+@pytest.mark.parametrize("keep", [True, False])
+@pytest.mark.parametrize("n,d,S,parts", [(296, 1024, 4, 0), (297, 1024, 4, 0), (445, 1032, 2, 9), (299, 2048, 3, 1), (1037, 2048, 4, 4), (300, 4096, 4, 4), (297, 4104, 4, 0)])
+def test_seam_over_streams_of_many_rows(n, d, S, parts, keep):
+    """Around the sizes of the persistent kernel: fewest rows and one less, the narrowest, a width that fills no warp, the widest and the next one; against 64 bits."""
+    g = torch.Generator().manual_seed(n + d)
+    r = lambda *s: torch.randn(*s, generator=g)
+    into, mix, out, w, eps = r(S) + 0.5, r(S, S) * 0.5, r(S), 1 + 0.3 * r(d), 1e-4
+    x0, y = r(n, S, d), (r(n, parts, d) if parts else r(n, d)).to(torch.bfloat16)
+    wt = torch.rand(n, parts, generator=g) if parts else None
+    x, h, st = _dev(x0), torch.zeros(n, d, dtype=torch.bfloat16, device="cuda"), _status()
+    R.stream_seam(x, n, h=h, norm=_dev(w), into=_dev(into), y=y.cuda(), parts_w=_dev(wt) if parts else None, mix=_dev(mix), out=_dev(out), keep=keep, eps=eps, status=st)
+    Y = (wt.double()[..., None] * y.double()).sum(1) if parts else y.double()
+    X = P.spread(x0.double().transpose(0, 1), mix.double(), out.double(), 1.0, Y)
+    H = P.rms(P.collapse(X, into.double()), w.double(), eps)
+    assert st.tolist()[0] == 0 and torch.equal(x.cpu(), x0) == (not keep)
+    if keep:
+        assert (x.transpose(0, 1).cpu().double() - X).abs().max() < 4e-6 * X.abs().max()
+    assert ((h.cpu().double() - H).abs() <= 2 ** -8 * H.abs() + 2e-5).all()
