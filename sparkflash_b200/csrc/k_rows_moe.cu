@@ -218,7 +218,12 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(PlanArgs a) {
   };
   for (int p0 = 0; p0 < a.pairs; p0 += BATCH * nt) places(p0);
   __syncthreads();
-  const int c = cnt[tid], t = (c + a.tile - 1) / a.tile;
+  const int c = cnt[tid];
+  int t = (c + a.tile - 1) / a.tile, per = a.tile;
+  if (a.tile > 128 && t) {  // tiles of two SMs (k_rows_moe_duo.cu): even ones, in the steps of that product's width
+    per = ((c + t - 1) / t + 63) / 64 * 64;
+    t = (c + per - 1) / per;
+  }
   int sc = c, st = t;       // inclusive sums of pairs and of tiles over the experts
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -228,7 +233,7 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(PlanArgs a) {
   if (lane == 31) { wsum[0][warp] = sc; wsum[1][warp] = st; }
   __syncthreads();
   for (int w = 0; w < warp; ++w) { sc += wsum[0][w]; st += wsum[1][w]; }
-  for (int k = 0; k < t; ++k) reinterpret_cast<int4*>(a.tiles)[st - t + k] = make_int4(tid, sc - c + k * a.tile, min(a.tile, c - k * a.tile), 0);
+  for (int k = 0; k < t; ++k) reinterpret_cast<int4*>(a.tiles)[st - t + k] = make_int4(tid, sc - c + k * per, min(per, c - k * per), 0);
   if (tid == nt - 1) *a.count = st;
   base[tid] = sc - c;
   cnt[tid] = 0;             // more pairs than the threads hold: they take their places again

@@ -690,16 +690,22 @@ class MixtureFF:
             R.moe_gemv(z, ids, wts, h, self.w_in, act, first, n, self.ff, top, slots, self.act, self.alpha, self.limit, self.choice)
             R.moe_gemv(None, ids, wts, act, self.w_out, parts, second, n, d, top, slots, None)
             return parts, wts
-        plan = (s.scratch.get("moe_order", n * top), s.scratch.get("moe_tiles", R.moe_tiles(n, self.E, top, self.tile), 4), s.scratch.get("moe_count", 4),
-                R.moe_tiles(n, self.E, top, self.tile))
+        duo = self.tc and R.moe_duo_takes(n, self.E, top, d, self.ff, self.act == "clamp")
+        tile = R.MOE_DUO_TILE if duo else self.tile
+        plan = (s.scratch.get("moe_order", n * top), s.scratch.get("moe_tiles", R.moe_tiles(n, self.E, top, tile), 4), s.scratch.get("moe_count", 4),
+                R.moe_tiles(n, self.E, top, tile))
         if n > R.MOE_PLAN_ROWS:
             R.moe_route(z, ids, wts, self.E, top, self.shared, self.choice)
-        R.moe_plan(z if n <= R.MOE_PLAN_ROWS else None, ids, wts, *plan[:3], self.E, top, self.shared, self.tile, self.choice)
+        R.moe_plan(z if n <= R.MOE_PLAN_ROWS else None, ids, wts, *plan[:3], self.E, top, self.shared, tile, self.choice)
         if self.tc:
             few, x = n <= R.MOE_GATHER_ROWS, h
             if not few:
                 x = s.scratch.get("moe_x", n * top, d)
                 R.moe_pick(h, plan[0], x, top)
+            if duo:
+                R.moe_duo(x, self.w_in, act, plan, first, n, self.ff, top, slots, self.act, s.status, self.alpha, self.limit)
+                R.moe_duo(act, self.w_out, parts, plan, second, n, d, top, slots, None, s.status)
+                return parts, wts
             R.moe_gemm(x, self.w_in, act, plan, first, n, self.ff, top, slots, self.act, s.status, self.alpha, self.limit, few)
             R.moe_gemm(act, self.w_out, parts, plan, second, n, d, top, slots, None, s.status)
             return parts, wts

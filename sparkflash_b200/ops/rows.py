@@ -583,6 +583,26 @@ def moe_gemm(x, w, out, plan, shared, n, M, top, slots, act, status, alpha=0.0, 
                                          c_int(gather), c_float(alpha), c_float(limit), c_float(sl), _p(status), _stream()), "rows_moe_gemm")
 
 
+MOE_DUO_TILE = 256         # pairs of a tile of two SMs (csrc/k_rows_moe_duo.cu)
+
+
+def moe_duo_takes(n: int, experts: int, top: int, width: int, ff: int, gated: bool) -> bool:
+    """Where two SMs on a tile are faster.  Both products, us, one SM against two, 32 experts: gated 4,096 / 2,048 wide, 64 pairs per expert 307 / 316, 128: 376 / 361,
+    250: 596 / 512, 512: 1,115 / 987; ungated 2,048 / 2,304, 375 pairs 224 / 192; gated 2,048 / 1,024, 512 pairs 330 / 375: a short sum leaves the
+    gates' way out, which takes longer than a tile of one SM's, uncovered."""
+    return n > MOE_GATHER_ROWS and n * top >= 128 * experts and min(width, ff) >= 2048 and (not gated or width >= 4096)
+
+
+def moe_duo(x, w, out, plan, shared, n, M, top, slots, act, status, alpha=0.0, limit=0.0):
+    """``moe_gemm`` with two SMs on a tile of up to 256 pairs; x in plan order."""
+    order, tiles, count, most = plan
+    sx, sw, sout, sm, sl = shared if shared is not None else (None, None, None, 0, 0.0)
+    msx, msw = (tensor_map(sx, sx.shape[1], 32).ptr, tensor_map(sw, sw.shape[1], 64).ptr) if shared is not None else (None, None)
+    _check(_lib.rows().sfb_rows_moe_duo(tensor_map(x, x.shape[1], 32).ptr, tensor_map(w, w.shape[2], 64).ptr, msx, msw, _p(order), _p(tiles), _p(count), _p(out), _p(sout),
+                                        c_int(most), c_int(n), c_int(M), c_int(w.shape[2]), c_int(sm), c_int(sw.shape[1] if sw is not None else 0), c_int(top),
+                                        c_int(slots), c_int(MOE_ACT[act]), c_float(alpha), c_float(limit), c_float(sl), _p(status), _stream()), "rows_moe_duo")
+
+
 def moe_gemv_takes(x: torch.Tensor, ff: int, shared_ff: int) -> bool:
     n, K = x.shape
     return x.dtype == torch.bfloat16 and n <= GEMV_ROWS and K % 8 == 0 and ff % 8 == 0 and shared_ff % 8 == 0 and max(K, ff, shared_ff) * 2 <= 200 * 1024

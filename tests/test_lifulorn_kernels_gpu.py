@@ -322,3 +322,51 @@ def test_all_rows_on_one_expert_and_close_calls(n):
     for j in range(2):
         want = P.expert(w64, f"e{j}.", h.double(), 2.0)
         assert (parts[:, j].double().cpu() - want).abs().max() < 2e-2 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("act", ["clamp", "relu2", "xielu"])
+@pytest.mark.parametrize("counts,d,ff,shared", [([257, 0, 64, 1], 64, 8, 0), ([256, 65, 128, 129, 63, 192], 72, 136, 72), ([513, 300, 511], 200, 264, 520), ([700], 1032, 128, 256)])
+def test_products_of_two_sms_are_those_of_one(counts, d, ff, shared, act):
+    """Tiles at and around their widths (64 pairs up to 256, cut evenly), widths and K that fill no tile, experts without a row: the bits of the kernel of one SM,
+    and the products in 64 bits (the first rounded to bf16 on its way into the second)."""
+    g = torch.Generator(device="cuda").manual_seed(sum(counts) + d)
+    r = lambda *s, by=1.0: (torch.randn(*s, device="cuda", generator=g) * by).to(torch.bfloat16)
+    n, E, gated, shared = sum(counts), len(counts), act == "clamp", shared if act == "clamp" else 0
+    x, w1, w2 = r(n, d), r(E, (1 + gated) * ff, d, by=d ** -0.5), r(E, d, ff, by=ff ** -0.5)
+    sw1, sw2 = (r(2 * shared, d, by=d ** -0.5), r(d, shared, by=shared ** -0.5)) if shared else (None, None)
+    ids = torch.cat([torch.full((c,), e, dtype=torch.int32) for e, c in enumerate(counts)])[torch.randperm(n, generator=torch.Generator().manual_seed(1))].cuda()[:, None].contiguous()
+    wts, alpha, limit, slots = torch.ones(n, 1 + bool(shared), device="cuda"), 1.2, 0.7, 1 + bool(shared)
+    got = {}
+    for tile, f in ((128, R.moe_gemm), (256, R.moe_duo)):
+        most, st = R.moe_tiles(n, E, 1, tile), _status()
+        order, tiles, count = torch.zeros(n, dtype=torch.int32, device="cuda"), torch.zeros(most, 4, dtype=torch.int32, device="cuda"), torch.zeros(4, dtype=torch.int32, device="cuda")
+        R.moe_plan(None, ids, wts, order, tiles, count, E, 1, int(bool(shared)), tile)
+        t = tiles[:int(count[0])].tolist()
+        assert [sum(p for x, _, p, _ in t if x == e) for e in range(E)] == counts and max(p for _, _, p, _ in t) <= tile
+        xp, a1 = torch.zeros(n, d, dtype=torch.bfloat16, device="cuda"), torch.full((n, ff), 9.0, dtype=torch.bfloat16, device="cuda")
+        sa, out = torch.full((n, max(8, shared)), 9.0, dtype=torch.bfloat16, device="cuda"), torch.full((n, slots, d), 9.0, dtype=torch.bfloat16, device="cuda")
+        R.moe_pick(x, order, xp, 1)
+        plan = (order, tiles, count, most)
+        f(xp, w1, a1, plan, (x, sw1, sa, shared, limit) if shared else None, n, ff, 1, slots, act, st, alpha, limit)
+        f(a1, w2, out, plan, (sa, sw2, None, d, 0.0) if shared else None, n, d, 1, slots, None, st)
+        assert st.tolist()[0] == 0
+        act1 = torch.zeros_like(a1)
+        act1[order.long()] = a1
+        got[tile] = (out, act1)
+    assert torch.equal(got[128][0], got[256][0]) and torch.equal(got[128][1], got[256][1])
+    def first(x, w, ff):
+        z = x @ w.t()
+        if gated:
+            a, u = z[:, :ff].clamp(max=limit), z[:, ff:].clamp(-limit, limit)
+            return a * torch.sigmoid(alpha * a) * (u + 1)
+        return z.clamp(min=0) ** 2 if act == "relu2" else torch.where(z > 0, alpha * z * z, limit * (torch.expm1(z.clamp(max=0)) - z)) + z / 2
+    for e in range(E):
+        rows = (ids[:, 0] == e).nonzero()[:, 0]
+        if len(rows):
+            h = first(x[rows].double(), w1[e].double(), ff)
+            assert ((got[256][1][rows].double() - h).abs() <= 2 ** -8 * h.abs() + 2e-3 * h.abs().max()).all()
+            y = got[256][1][rows].double() @ w2[e].double().t()
+            assert ((got[256][0][rows, 0].double() - y).abs() <= 2 ** -8 * y.abs() + 1e-5 * y.abs().max()).all()
+    if shared:
+        y = first(x.double(), sw1.double(), shared).to(torch.bfloat16).double() @ sw2.double().t()
+        assert ((got[256][0][:, 1].double() - y).norm() / y.norm()) < 5e-3
