@@ -215,6 +215,12 @@ int sfb_rope_table(const double* const* inv_freq, const int* ratio, int V, int h
   return (int)sfb_launch(rope_table_kernel, dim3(n), dim3(128), 0, stream, a);
 }
 
+// `planes` runs of `bytes` bytes, `pitch` bytes apart on both sides, from host to device
+int sfb_copy_planes(void* dst, const void* src, int64_t pitch, int64_t bytes, int planes, cudaStream_t stream) {
+  if (pitch < 1 || bytes < 1 || bytes > pitch || planes < 1) return (int)cudaErrorInvalidValue;
+  return (int)cudaMemcpy2DAsync(dst, (size_t)pitch, src, (size_t)pitch, (size_t)bytes, (size_t)planes, cudaMemcpyHostToDevice, stream);
+}
+
 int sfb_prefetch_l2(const void* p, int64_t bytes, cudaStream_t stream) {
   if (bytes <= 0) return 0;
   const int64_t threads = (bytes + 2047) / 2048;

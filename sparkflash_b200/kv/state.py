@@ -13,7 +13,7 @@ from dataclasses import dataclass, field
 import torch
 
 
-@dataclass
+@dataclass(slots=True)
 class _Lane:
     rows: int = 0                 # positions the current version stands for
     version: int = 0
@@ -22,7 +22,7 @@ class _Lane:
     tokens: list[int] = field(default_factory=list)      # ... and the tokens it ran
 
 
-@dataclass
+@dataclass(slots=True)
 class Advance:
     """One segment's part in a step: read slot ``src``, write slot ``dst``, after running ``replay`` tokens again first."""
     lane: int

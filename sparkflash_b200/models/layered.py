@@ -21,6 +21,7 @@ import gc
 import json
 import os
 import warnings
+from array import array
 
 import numpy as np
 import torch
@@ -242,7 +243,14 @@ class LayeredEngine:
             seen.add(lane)
             segs.append((lane, p0, tokens[i:j], i))
             i = j
-        if min(tokens) < 0 or max(tokens) >= self.model.vocab:
+        try:
+            self._tokens = np.frombuffer(array("i", tokens), np.int32)         # for _stage; a list of thousands is gone through once
+        except TypeError:                  # numbers that are no integers are cut
+            inside = min(tokens) >= 0 and max(tokens) < self.model.vocab
+            self._tokens = np.fromiter(tokens, np.int32, n) if inside else np.array([-1], np.int32)
+        except OverflowError:
+            self._tokens = np.array([-1], np.int32)
+        if self._tokens.min() < 0 or self._tokens.max() >= self.model.vocab:
             bad = [t for t in tokens if not 0 <= t < self.model.vocab]
             raise ValueError(f"token {bad[0]} outside the vocabulary of {self.model.vocab}")
         return segs
@@ -292,8 +300,8 @@ class LayeredEngine:
         if s.single:
             rows_tok[:], rows_pos[:], rows_lane[:] = [r[0] for r in runs], [a.start for a in advs], [seg[0] for seg in segs]
         else:
-            for (lane, _, _, _), adv, run, r, m in zip(segs, advs, runs, row0, length):
-                rows_tok[r:r + m] = np.fromiter(run, np.int32, m)
+            for (lane, _, _, i), adv, run, r, m in zip(segs, advs, runs, row0, length):
+                rows_tok[r:r + m] = np.fromiter(run, np.int32, m) if adv.replay else self._tokens[i:i + m]
                 rows_pos[r:r + m] = np.arange(adv.start, adv.start + m, dtype=np.int32)
                 rows_lane[r:r + m] = lane
         hpos[:] = rows_pos if all_heads else rows_pos[hrows]
@@ -374,25 +382,28 @@ class LayeredEngine:
         n = len(tokens)
         if self._event is not None:
             self._event.synchronize()         # the previous step's copies have left the pinned buffers
-        segs = self._segments(tokens, lanes, positions)
-        heads = list(range(n)) if head is True else [] if head is False else [n - 1] if head == "last" else list(head)
-        advs = [self.state.plan(lane, p0) for lane, p0, _, _ in segs]
-        for (lane, p0, toks, _), adv in zip(segs, advs):
-            self.kv.ensure(lane, p0 + len(toks))
         graphs = self.use_graphs and not masks and self.tap_layers is None
-        s = self._stage(segs, advs, heads, temperature, seeds, bool(sample) if graphs else None)
-        mask = self._stage_masks(masks, heads) if masks else None
-        if s.graph is not None:
-            self._replay(s, bool(sample))
-        else:
-            self._run(s, sample, mask)
-        for (lane, p0, toks, _), adv in zip(segs, advs):
-            self.state.commit(adv, adv.replay + toks if adv.replay else toks)
+        whole, mask, heads = True, None, range(n)
+        if not (graphs and head is True and self._continue(tokens, lanes, positions, temperature, seeds, bool(sample))):
+            segs = self._segments(tokens, lanes, positions)
+            heads = list(range(n)) if head is True else [] if head is False else [n - 1] if head == "last" else list(head)
+            advs = [self.state.plan(lane, p0) for lane, p0, _, _ in segs]
+            for (lane, p0, toks, _), adv in zip(segs, advs):
+                self.kv.ensure(lane, p0 + len(toks))
+            s = self._stage(segs, advs, heads, temperature, seeds, bool(sample) if graphs else None)
+            mask = self._stage_masks(masks, heads) if masks else None
+            if s.graph is not None:
+                self._replay(s, bool(sample))
+            else:
+                self._run(s, sample, mask)
+            for (lane, p0, toks, _), adv in zip(segs, advs):
+                self.state.commit(adv, adv.replay + toks if adv.replay else toks)
+            whole = s.whole
         if not sample or not heads or not sync:
             return self.best_id[:len(heads)] if sample and heads else None if not sync else torch.zeros((n,), dtype=torch.int32)
         self._out[:len(heads)].copy_(self.best_id[:len(heads)], non_blocking=True)
         torch.cuda.current_stream().synchronize()
-        if s.whole:
+        if whole:
             out = self._out[:n].clone()
         else:
             out = torch.zeros((n,), dtype=torch.int32)
@@ -402,6 +413,53 @@ class LayeredEngine:
             lg = self.logits[k] if mask is None else self.logits[k].masked_fill(mask[k] == 0, float("-inf"))
             out[r] = candidate_choice(lg, 0, 1, top_k, top_p, float(temperature[r]), int(seeds[r]) if seeds is not None else 0, positions[r])
         return out
+
+    def _continue(self, tokens, lanes, positions, temps, seeds, sample: bool) -> bool:
+        """The step of a decoding server - one row for each of several lanes, next to what the lane holds, its first, or its latest again, every row with
+        a head - where it has been captured: checked, staged as ``_stage`` does and replayed, with nothing made per row but numbers.  False: another
+        step, or not captured yet; nothing has changed.  (Ahead of the replay 64 / 16 / 1 rows take 52 / 36 / 28 us, through
+        segments and their advances 118 / 64 / 40.)"""
+        tokens, lanes, positions = (x if type(x) is list else list(x) for x in (tokens, lanes, positions))
+        n, held, pages = len(tokens), self.state.lanes, self.kv.pages
+        if not n or not n == len(lanes) == len(positions) == len(set(lanes)):
+            return False
+        top = max(positions)
+        graph = self.graphs.get((n, _bucket(top // PAGE + 1), sample))
+        if graph is None or min(lanes) < 0 or max(lanes) >= self.max_lanes or min(positions) < 0 or top >= self.max_context or min(tokens) < 0 or max(tokens) >= self.vocab:
+            return False
+        src, dst = [], []
+        for lane, pos in zip(lanes, positions):      # as StateSlots.plan
+            s = held[lane]
+            if not pos or pos == s.rows:
+                src.append(2 * lane + s.version if pos else -1)
+                dst.append(2 * lane + (s.version ^ 1))
+            elif pos == s.start and pos < s.rows:
+                src.append(s.start_slot)
+                dst.append(2 * lane + s.version)
+            else:
+                return False
+        for lane, pos in zip(lanes, positions):
+            if len(pages[lane]) * PAGE <= pos:
+                self.kv.ensure(lane, pos + 1)
+        words = [0] * (2 * n) if seeds is None else [w for i in range(n) for w in _words(seeds[i])]
+        words += [0] * n if temps is None else [_float_bits(temps[i]) for i in range(n)]
+        words += positions + tokens + positions + lanes + src + dst
+        try:
+            staged = array("i", words)
+        except TypeError:
+            return False
+        at = len(words)
+        self._np[:at] = staged
+        self._meta[:at].copy_(self._host[:at], non_blocking=True)
+        self.kv.upload()
+        if self._event is not None:
+            self._event.record()
+        self.logits = self.scratch.get("logits", n, self.vocab)
+        graph.replay()
+        for lane, pos, tok, old, new in zip(lanes, positions, tokens, src, dst):
+            s = held[lane]
+            s.start, s.start_slot, s.tokens, s.rows, s.version = pos, old, [tok], pos + 1, new & 1
+        return True
 
     def _run(self, s: Step, sample: bool = True, mask=None) -> None:
         with R.exact_matmul():

@@ -275,6 +275,11 @@ def rope_table(inv_freqs, ratios, row_pos, out, n):
            "rope_table")
 
 
+def copy_planes(dst, src, n):
+    """The first n elements of every plane of ``src`` [planes, rows] (pinned) to ``dst`` (device, the same shape), in one copy on the current stream."""
+    _check(lib().sfb_copy_planes(_p(dst), _p(src), c_int64(dst.stride(0) * dst.element_size()), c_int64(n * dst.element_size()), c_int(dst.shape[0]), _stream()), "copy_planes")
+
+
 def prefetch_l2(t: torch.Tensor):
     _check(lib().sfb_prefetch_l2(_p(t), c_int64(t.numel() * t.element_size()), _stream()), "prefetch_l2")
 

@@ -180,3 +180,44 @@ def test_runs_of_a_lane_end_where_the_next_one_begins(runs):
 def test_rows_that_make_no_step_are_refused(engine, tokens, lanes, positions, message):
     with pytest.raises(ValueError, match=message):
         engine.step(tokens, lanes, positions)
+
+
+@pytest.mark.parametrize("kind", [list, tuple, np.array])
+def test_a_continued_step_is_staged_as_any_other(engine, kind):
+    """Captured steps of one row per lane through the short way and through segments: the same index buffer, pages, states, errors and answers, for rows
+    that go on, begin again at 0, repeat the latest position or are none of these."""
+    other = LY.LayeredEngine(_Model(), max_lanes=4, max_context=512, max_rows=64)
+    other._continue = lambda *a: False
+    rng, short = random.Random(5), 0
+    engine._continue = lambda *a, go=engine._continue: go(*a) and (setattr(engine, "taken", engine.taken + 1) or True)
+    engine.taken = 0
+    staged = {}
+
+    def replay(e):
+        staged[e] = e._meta[:9 * len(lanes)].tolist()
+        e.best_id[:len(lanes)] = e._meta[3 * len(lanes):4 * len(lanes)] + 1000
+    for e in (engine, other):
+        e.graphs.update({(n, b, s): SimpleNamespace(replay=lambda e=e: replay(e)) for n in range(1, 5) for b in (16,) for s in (True, False)})
+        for lane in range(4):
+            lanes = [lane] * (40 + lane)
+            e.step([1] * len(lanes), lanes, list(range(len(lanes))), head=False)
+    for turn in range(150):
+        lanes = rng.sample(range(4), rng.randint(1, 4))
+        rows = [engine.state.lanes[lane] for lane in lanes]
+        pos = [0 if rng.random() < 0.05 else s.start if rng.random() < 0.2 else s.rows + (rng.random() < 0.02) for s in rows]
+        toks = [rng.randrange(VOCAB + (rng.random() < 0.02)) for _ in lanes]
+        kw = dict(temperature=rng.choice([None, [rng.random() for _ in lanes]]), seeds=rng.choice([None, [rng.getrandbits(64) - 2 ** 63 for _ in lanes]]), sample=rng.random() < 0.8)
+        got = []
+        for e in (engine, other):
+            staged[e] = None
+            try:
+                got.append(e.step(kind(toks), kind(lanes), kind(pos), **kw).tolist())
+            except ValueError as x:
+                got.append(str(x))
+        assert got[0] == got[1] and staged[engine] == staged[other], turn
+        assert [vars_of(s) for s in engine.state.lanes] == [vars_of(s) for s in other.state.lanes] and engine.kv.pages == other.kv.pages, turn
+    assert engine.taken > 75
+
+
+def vars_of(lane):
+    return lane.rows, lane.version, lane.start, lane.start_slot, list(lane.tokens)
