@@ -70,6 +70,23 @@ def test_seam_norms_merge_embedding_and_step_vector(dt, d):
     assert st.tolist()[0] == 2 and st.tolist()[2] == V          # a token outside the table is reported, not read
 
 
+@pytest.mark.parametrize("dt", DTYPES)
+@pytest.mark.parametrize("d", [1024, 1036, 2048, 4096])
+def test_seam_of_decoded_rows_of_eight_warps(dt, d):
+    """Widths whose rows are eight warps of a decode step's block (and one that is nine): both norms' moments, against 64 bits."""
+    g = torch.Generator().manual_seed(d)
+    n, eps = 3, 1e-4
+    x, y = torch.randn(n, d, generator=g), (torch.randn(n, d, generator=g) + 1).to(dt)
+    w, b = [1 + 0.3 * torch.randn(d, generator=g) for _ in range(2)], [0.3 * torch.randn(d, generator=g) for _ in range(2)]
+    ln = lambda t, a, o: torch.nn.functional.layer_norm(t, (d,), a.double(), o.double(), eps)
+    want_x = x.double() + ln(y.double(), w[0], b[0])
+    want_h = ln(want_x, w[1], b[1])
+    X, H, st = x.cuda(), torch.zeros(n, d, dtype=dt, device="cuda"), _status()
+    R.seam(X, n, h=H, y=y.cuda(), post=(w[0].cuda(), b[0].cuda()), norm=(w[1].cuda(), b[1].cuda()), eps=eps, status=st)
+    assert st.tolist()[0] == 0 and (X.cpu().double() - want_x).abs().max() < 2e-5
+    assert ((H.cpu().double() - want_h).abs() <= (2 ** -8 if dt == torch.bfloat16 else 0) * want_h.abs() + 4e-5).all()
+
+
 @pytest.mark.parametrize("form", ["layer", "rms", "scale", "plain", "merged", "parts1", "parts9", "norm"])
 @pytest.mark.parametrize("n,d", [(296, 2048), (297, 2048), (445, 2056), (1037, 3000), (299, 4096), (297, 4104), (2048, 1024), (2047, 1024), (2050, 1032), (400, 264)])
 def test_seam_of_many_rows(n, d, form):
